@@ -4,7 +4,7 @@
  * The reference (hustvl/MoDA) has no native layer: its operators are Python functions
  * that launch Triton kernels.  Each entry point below names the reference function
  * whose device work it replaces; the Python mirror of those functions
- * (moda_b200/ops.py) binds this library with ctypes.
+ * (moda_b200/ops.py) binds this library through moda_b200/csrc/torch_binding.cpp and ctypes.
  *
  * Conventions
  *   - Tensors are 4-D [B, T, H, D] with arbitrary element strides for B, T, H and a
@@ -197,6 +197,16 @@ int moda_b200_bwd_static_scratch(const moda_problem *prob, const moda_tensor4 *q
 int moda_b200_depth_append(const moda_problem *prob, const moda_tensor4 *k, const moda_tensor4 *v,
                            const moda_tensor4 *cache_k, const moda_tensor4 *cache_v, int32_t layer,
                            void *stream);
+
+/*
+ * The way back, for the gradients of a layer cache: copies slot `layer` of the gradient caches
+ * grad_k / grad_v ([B, T_kv*Lmax, H, D]) into d_k and d_v ([B, T_kv, H, D]).  Same fields of
+ * `prob` and the same checks as moda_b200_depth_append.  Replaces the un-stacking of the depth
+ * gradients in the reference caller's backward.
+ */
+int moda_b200_depth_take(const moda_problem *prob, const moda_tensor4 *grad_k,
+                         const moda_tensor4 *grad_v, int32_t layer, const moda_tensor4 *d_k,
+                         const moda_tensor4 *d_v, void *stream);
 
 /*
  * Validation only (no launch): the status moda_b200_fwd / moda_b200_bwd would return

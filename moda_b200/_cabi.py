@@ -1,4 +1,5 @@
-"""ctypes binding of ``libmoda_b200.so`` (declarations: ``include/moda_b200.h``).
+"""Binding of ``libmoda_b200.so`` (declarations: ``include/moda_b200.h``): ctypes for everything that is
+not on the path of an operator call, and the native module (``csrc/torch_binding.cpp``) for what is.
 
 The library is the only compute path of this package: there is no eager / CPU
 fallback.  Loading fails loudly when the shared object has not been built
@@ -27,6 +28,7 @@ EXPORTED_SYMBOLS = (
     "moda_b200_bwd",
     "moda_b200_bwd_static_scratch",
     "moda_b200_depth_append",
+    "moda_b200_depth_take",
     "moda_b200_check_problem",
     "moda_b200_resolve_path",
     "moda_b200_profile_begin",
@@ -101,6 +103,8 @@ def load() -> ctypes.CDLL:
     lib.moda_b200_bwd_static_scratch.restype = ctypes.c_int
     lib.moda_b200_depth_append.argtypes = [P, T, T, T, T, ctypes.c_int32, V]
     lib.moda_b200_depth_append.restype = ctypes.c_int
+    lib.moda_b200_depth_take.argtypes = [P, T, T, ctypes.c_int32, T, T, V]
+    lib.moda_b200_depth_take.restype = ctypes.c_int
     lib.moda_b200_check_problem.argtypes = [P]
     lib.moda_b200_check_problem.restype = ctypes.c_int
     lib.moda_b200_resolve_path.argtypes = [P, ctypes.c_int]
@@ -122,6 +126,24 @@ def load() -> ctypes.CDLL:
     lib.moda_b200_version.restype = ctypes.c_int
     _lib = lib
     return lib
+
+
+_native = None
+
+
+def native():
+    """The native binding module, with this module's errors hooked up."""
+    global _native
+    if _native is None:
+        load()
+        try:
+            from . import _native as mod
+        except ImportError as e:
+            raise ModaLibraryError(f"moda_b200/_native.so cannot be loaded ({e}): build it with "
+                                   "`python -m moda_b200.build` (there is no fallback path)") from e
+        mod.set_check(check)
+        _native = mod
+    return _native
 
 
 def status_string(status: int) -> str:

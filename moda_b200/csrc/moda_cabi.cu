@@ -195,7 +195,6 @@ Params sequence_part(const Params& p) {
   s.merge_depth = 1;
   return s;
 }
-
 template <typename T, int D>
 int fda_fwd(const Params& p, int n_sm, cudaStream_t st) {
   const int64_t units = (int64_t)p.B * p.T_kv * p.H;
@@ -274,6 +273,39 @@ struct DeviceGuard {
   }
   ~DeviceGuard() { int cur = -1; if (cudaGetDevice(&cur) == cudaSuccess && cur != prev && prev >= 0) cudaSetDevice(prev); }
 };
+
+// One layer's rows into (kTake: out of) slot `layer` of the caches.
+template <bool kTake>
+int cache_slot(const moda_problem* prob, const moda_tensor4* k, const moda_tensor4* v, const moda_tensor4* cache_k,
+               const moda_tensor4* cache_v, int32_t layer, void* stream) {
+  if (prob == nullptr) return MODA_ERR_NULL;
+  if (prob->B < 1 || prob->T_kv < 1 || prob->H < 1 || prob->B > 65535 || prob->H > 65535) return MODA_ERR_SHAPE;
+  if (prob->D != 64 && prob->D != 128) return MODA_ERR_HEAD_DIM;
+  if (prob->dtype != MODA_BF16 && prob->dtype != MODA_FP16) return MODA_ERR_DTYPE;
+  const int Lmax = prob->depth_rows_per_pos;
+  if (Lmax < 1 || layer < 0 || layer >= Lmax || (int64_t)prob->T_kv * Lmax > (int64_t)1 << 30) return MODA_ERR_SHAPE;
+  if (int rc = check_tensor(k, true, prob->B, prob->T_kv, prob->H)) return rc;
+  if (int rc = check_tensor(v, true, prob->B, prob->T_kv, prob->H)) return rc;
+  if (int rc = check_tensor(cache_k, true, prob->B, (int64_t)prob->T_kv * Lmax, prob->H)) return rc;
+  if (int rc = check_tensor(cache_v, true, prob->B, (int64_t)prob->T_kv * Lmax, prob->H)) return rc;
+  DeviceGuard guard(prob->device);
+  if (!guard.ok) return cuda_fail(guard.err);
+  g_last_launches = 0;
+  const int n_sm = sm_count(prob->device);
+  if (n_sm <= 0) return cuda_fail(cudaErrorInvalidDevice);
+  cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
+  const int64_t n = (int64_t)prob->B * prob->T_kv * prob->H * (prob->D / 8);
+  const int64_t want = (n + 255) / 256, cap = (int64_t)n_sm * 16;
+  const int blocks = (int)(want < cap ? want : cap);
+  {
+    prof::Scope ps(prof::kDepthAppend, st);
+    auto kern = prob->D == 128 ? cache::slot_kernel<16, kTake> : cache::slot_kernel<8, kTake>;
+    kern<<<blocks, 256, 0, st>>>(to_view(k), to_view(v), to_view(cache_k), to_view(cache_v), prob->B, prob->T_kv, prob->H, Lmax, layer);
+  }
+  MODA_CUDA(cudaGetLastError());
+  g_last_launches += 1;
+  return MODA_OK;
+}
 
 }  // namespace
 
@@ -410,37 +442,11 @@ int moda_b200_bwd(const moda_problem* prob, const moda_tensor4* q, const moda_te
 
 int moda_b200_depth_append(const moda_problem* prob, const moda_tensor4* k, const moda_tensor4* v,
                            const moda_tensor4* cache_k, const moda_tensor4* cache_v, int32_t layer, void* stream) {
-  if (prob == nullptr) return MODA_ERR_NULL;
-  if (prob->B < 1 || prob->T_kv < 1 || prob->H < 1 || prob->B > 65535 || prob->H > 65535) return MODA_ERR_SHAPE;
-  if (prob->D != 64 && prob->D != 128) return MODA_ERR_HEAD_DIM;
-  if (prob->dtype != MODA_BF16 && prob->dtype != MODA_FP16) return MODA_ERR_DTYPE;
-  const int Lmax = prob->depth_rows_per_pos;
-  if (Lmax < 1 || layer < 0 || layer >= Lmax || (int64_t)prob->T_kv * Lmax > (int64_t)1 << 30) return MODA_ERR_SHAPE;
-  if (int rc = check_tensor(k, true, prob->B, prob->T_kv, prob->H)) return rc;
-  if (int rc = check_tensor(v, true, prob->B, prob->T_kv, prob->H)) return rc;
-  if (int rc = check_tensor(cache_k, true, prob->B, (int64_t)prob->T_kv * Lmax, prob->H)) return rc;
-  if (int rc = check_tensor(cache_v, true, prob->B, (int64_t)prob->T_kv * Lmax, prob->H)) return rc;
-  DeviceGuard guard(prob->device);
-  if (!guard.ok) return cuda_fail(guard.err);
-  g_last_launches = 0;
-  const int n_sm = sm_count(prob->device);
-  if (n_sm <= 0) return cuda_fail(cudaErrorInvalidDevice);
-  cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-  const int64_t n = (int64_t)prob->B * prob->T_kv * prob->H * (prob->D / 8);
-  const int64_t want = (n + 255) / 256, cap = (int64_t)n_sm * 16;
-  const int blocks = (int)(want < cap ? want : cap);
-  {
-    prof::Scope ps(prof::kDepthAppend, st);
-    if (prob->D == 128)
-      cache::append_kernel<16><<<blocks, 256, 0, st>>>(to_view(k), to_view(v), to_view(cache_k), to_view(cache_v),
-                                                      prob->B, prob->T_kv, prob->H, Lmax, layer);
-    else
-      cache::append_kernel<8><<<blocks, 256, 0, st>>>(to_view(k), to_view(v), to_view(cache_k), to_view(cache_v),
-                                                     prob->B, prob->T_kv, prob->H, Lmax, layer);
-  }
-  MODA_CUDA(cudaGetLastError());
-  g_last_launches += 1;
-  return MODA_OK;
+  return cache_slot<false>(prob, k, v, cache_k, cache_v, layer, stream);
+}
+int moda_b200_depth_take(const moda_problem* prob, const moda_tensor4* grad_k, const moda_tensor4* grad_v, int32_t layer,
+                         const moda_tensor4* d_k, const moda_tensor4* d_v, void* stream) {
+  return cache_slot<true>(prob, d_k, d_v, grad_k, grad_v, layer, stream);
 }
 
 int moda_b200_profile_begin(void) {

@@ -51,6 +51,7 @@ def set_kernel_path(path: int) -> int:
     """Force PATH_AUTO / PATH_SIMT_MMA / PATH_TCGEN05 for subsequent calls; returns the old value."""
     global _forced_path
     old, _forced_path = _forced_path, int(path)
+    _cabi.native().set_path(_forced_path)
     return old
 
 
@@ -73,89 +74,35 @@ def _ref(t: Optional[Tensor4]):
     return ctypes.byref(t) if t is not None else None
 
 
-def _problem(q, T_kv, L, G, mode, scale, chunk_rows, depth_rows_per_pos=0, accumulate_depth_grads=0) -> Problem:
+def _check_tensors(q, *others):
     if not q.is_cuda:
         raise RuntimeError("moda_b200 runs on CUDA tensors only (there is no CPU path)")
     if q.dtype not in _DTYPES:
         raise TypeError(f"moda_b200 supports bf16/fp16 inputs, got {q.dtype}")
-    B, T_q, H, D = q.shape
-    return Problem(B, T_kv, H, D, G, L, mode, chunk_rows, _DTYPES[q.dtype], _forced_path,
-                   float(scale), q.device.index if q.device.index is not None else torch.cuda.current_device(),
-                   int(depth_rows_per_pos), int(accumulate_depth_grads))
-
-
-def _check_same(q, *others):
     for x in others:
         if x is not None:
             assert x.dtype == q.dtype and x.device == q.device, "all tensors must share dtype and device"
 
 
-def _forward(q, k, v, cached_k, cached_v, scale, G, mode, chunk_rows=CHUNK_VISIBLE_QUERY_ROWS,
-             cache_layers=None, cache_capacity=0):
-    """``cache_layers`` / ``cache_capacity``: cached_k / cached_v are an in-place layer cache
-    ``[B, T_kv*capacity, H, D]`` of which the first ``cache_layers`` layers are valid."""
+def _problem(q, T_kv, L, G, mode, scale, chunk_rows) -> Problem:
+    _check_tensors(q)
     B, T_q, H, D = q.shape
-    assert T_q % G == 0, "T_q must be divisible by moda_group_num"
-    T_kv = T_q // G
-    use_depth = cached_k is not None and cached_v is not None
-    L = (cached_k.shape[1] // T_kv if cache_layers is None else cache_layers) if use_depth else 0
-    _check_same(q, k, v, cached_k, cached_v)
-    q, k, v, cached_k, cached_v = [None if x is None else _usable(x) for x in (q, k, v, cached_k, cached_v)]
-    if not use_depth:
-        cached_k = cached_v = None
-    prob = _problem(q, T_kv, L, G, mode, scale, chunk_rows, cache_capacity)
-    o = torch.empty(B, T_q, H, D, dtype=q.dtype, device=q.device)
-    lse = torch.empty(B, T_q, H, dtype=torch.float32, device=q.device)
-    lib = _cabi.load()
-    tq, tk, tv, tkd, tvd, to = map(_t4, (q, k, v, cached_k, cached_v, o))
-    with torch.cuda.device(q.device):
-        stream = torch.cuda.current_stream().cuda_stream
-        rc = lib.moda_b200_fwd(ctypes.byref(prob), _ref(tq), _ref(tk), _ref(tv), _ref(tkd), _ref(tvd),
-                               _ref(to), lse.data_ptr(), stream)
-    _cabi.check(rc, "moda_b200_fwd")
-    return o, lse
+    return Problem(B, T_kv, H, D, G, L, mode, chunk_rows, _DTYPES[q.dtype], _forced_path,
+                   float(scale), q.device.index if q.device.index is not None else torch.cuda.current_device(), 0, 0)
 
 
-def _backward(q, k, v, cached_k, cached_v, o, lse, do, scale, G, mode,
-              chunk_rows=CHUNK_VISIBLE_QUERY_ROWS, cache_layers=None, cache_capacity=0, grad_cache=None):
-    """``cache_layers`` / ``cache_capacity`` as in ``_forward``; ``grad_cache = (gk, gv)``: gradient
-    caches of the same layout to which the depth gradients are ADDED (the returned depth gradients
-    are then those tensors)."""
-    B, T_q, H, D = q.shape
-    T_kv = T_q // G
-    use_depth = cached_k is not None and cached_v is not None
-    L = (cached_k.shape[1] // T_kv if cache_layers is None else cache_layers) if use_depth else 0
-    _check_same(q, k, v, cached_k, cached_v, o, do)
-    q, k, v, cached_k, cached_v, o, do = [
-        None if x is None else _usable(x) for x in (q, k, v, cached_k, cached_v, o, do)]
-    if not use_depth:
-        cached_k = cached_v = None
-    lse = lse.contiguous()
+def _forward(q, k, v, cached_k, cached_v, scale, G, mode, chunk_rows=CHUNK_VISIBLE_QUERY_ROWS):
+    """(o, lse), no autograd."""
+    assert q.shape[1] % G == 0, "T_q must be divisible by moda_group_num"
+    _check_tensors(q, k, v, cached_k, cached_v)
+    return _cabi.native().forward(q, k, v, cached_k, cached_v, scale, G, mode, chunk_rows)
+
+
+def _backward(q, k, v, cached_k, cached_v, o, lse, do, scale, G, mode, chunk_rows=CHUNK_VISIBLE_QUERY_ROWS):
+    """(dq, dk, dv, d_cached_k, d_cached_v), None where there is no such input."""
+    _check_tensors(q, k, v, cached_k, cached_v, o, do)
     assert lse.dtype == torch.float32
-    prob = _problem(q, T_kv, L, G, mode, scale, chunk_rows, cache_capacity, 1 if grad_cache is not None else 0)
-    dq = torch.empty_like(q, memory_format=torch.contiguous_format)
-    dk = torch.empty_like(k, memory_format=torch.contiguous_format) if k is not None else None
-    dv = torch.empty_like(v, memory_format=torch.contiguous_format) if v is not None else None
-    if grad_cache is not None:
-        dkd, dvd = grad_cache
-        assert use_depth and dkd.shape == cached_k.shape and dvd.shape == cached_v.shape
-        assert _usable(dkd) is dkd and _usable(dvd) is dvd
-    else:
-        dkd = torch.empty_like(cached_k, memory_format=torch.contiguous_format) if use_depth else None
-        dvd = torch.empty_like(cached_v, memory_format=torch.contiguous_format) if use_depth else None
-    lib = _cabi.load()
-    nbytes = ctypes.c_size_t(0)
-    _cabi.check(lib.moda_b200_bwd_workspace_bytes(ctypes.byref(prob), ctypes.byref(nbytes)),
-                "moda_b200_bwd_workspace_bytes")
-    ws = torch.empty(max(int(nbytes.value), 256), dtype=torch.uint8, device=q.device)
-    ts = list(map(_t4, (q, k, v, cached_k, cached_v, o)))
-    gs = list(map(_t4, (do, dq, dk, dv, dkd, dvd)))
-    with torch.cuda.device(q.device):
-        stream = torch.cuda.current_stream().cuda_stream
-        rc = lib.moda_b200_bwd(ctypes.byref(prob), *[_ref(t) for t in ts], lse.data_ptr(),
-                               *[_ref(t) for t in gs], ws.data_ptr(), ws.numel(), stream)
-    _cabi.check(rc, "moda_b200_bwd")
-    return dq, dk, dv, dkd, dvd
+    return _cabi.native().backward(q, k, v, cached_k, cached_v, o, lse, do, scale, G, mode, chunk_rows)
 
 
 def last_launch_count() -> int:
@@ -176,29 +123,10 @@ def tensor_pipe_rates(device=None) -> dict:
     return dict(zip(_cabi.TENSOR_PIPE_SHAPES, vals))
 
 
-# --------------------------------------------------------------------------- autograd
-class _ModaFunction(torch.autograd.Function):
-    """Autograd glue (reference: moda_v14.py:2649-2789, moda_v16.py:3320-3493,
-    fda_v12.py:1207-1338).  Saves inputs, o and lse; ``dlse`` is ignored like the
-    reference (moda_v14.py:2727)."""
-
-    @staticmethod
-    def forward(ctx, q, k, v, cached_k, cached_v, scale, G, mode):
-        o, lse = _forward(q, k, v, cached_k, cached_v, scale, G, mode)
-        ctx.save_for_backward(q, k, v, cached_k, cached_v, o, lse)
-        ctx.scale, ctx.G, ctx.mode = scale, G, mode
-        ctx.mark_non_differentiable(lse)
-        return o, lse
-
-    @staticmethod
-    def backward(ctx, do, dlse_unused):
-        q, k, v, cached_k, cached_v, o, lse = ctx.saved_tensors
-        dq, dk, dv, dkd, dvd = _backward(q, k, v, cached_k, cached_v, o, lse, do.to(q.dtype),
-                                         ctx.scale, ctx.G, ctx.mode)
-        return dq, dk, dv, dkd, dvd, None, None, None
-
-
 # --------------------------------------------------------------------------- wrappers
+# A call that is well-formed (the native binding checks it: layout, types, shapes, nothing to warn
+# about) goes straight to the kernels; anything else takes _prepare, which transposes, warns or says
+# what is wrong.
 def _prepare(api, q, k, v, g, cached_k, cached_v, scale, G, head_first, return_depth_grads,
              warn_shape, cu_seqlens, need_kv=True):
     assert g is None, f"{api}: gating (g) is not supported on the MoDA path"            # moda_v14.py:2672
@@ -248,6 +176,14 @@ def _prepare(api, q, k, v, g, cached_k, cached_v, scale, G, head_first, return_d
     return q, k, v, cached_k, cached_v, float(scale)
 
 
+def _attention(q, k, v, cached_k, cached_v, scale, G, mode):
+    """The differentiable operator on arguments that ``_prepare`` has looked at: o, lse in base-2 units
+    (not differentiable: its gradient is ignored like the reference's, moda_v14.py:2727); autograd glue
+    of moda_v14.py:2649-2789, moda_v16.py:3320-3493 and fda_v12.py:1207-1338."""
+    _check_tensors(q, k, v, cached_k, cached_v)
+    return _cabi.native().attention(q, k, v, cached_k, cached_v, scale, G, mode, True, False, True)
+
+
 def parallel_moda(q, k, v, g=None, cached_k=None, cached_v=None, scale=None, cu_seqlens=None,
                   moda_group_num=1, is_causal=True, head_first=False, need_lse=False,
                   return_depth_grads=True, warn_shape=True, customized_BT=None, customized_BS=None,
@@ -258,11 +194,16 @@ def parallel_moda(q, k, v, g=None, cached_k=None, cached_v=None, scale=None, cu_
     Returns ``o`` ([B,T_q,H,D], q.dtype) or ``(o, lse)`` (lse fp32, base-2) when
     ``need_lse``.  Outputs stay in the reference's layout (also for ``head_first``:
     the reference does not transpose back)."""
+    mode = MODE_CAUSAL if is_causal else MODE_NONCAUSAL
+    if g is None and cu_seqlens is None and not head_first:
+        r = _cabi.native().attention(q, k, v, cached_k, cached_v, scale, moda_group_num, mode,
+                                     return_depth_grads, warn_shape, False)
+        if r is not None:
+            return r if need_lse else r[0]
     q, k, v, cached_k, cached_v, scale = _prepare(
         "parallel_moda", q, k, v, g, cached_k, cached_v, scale, moda_group_num, head_first,
         return_depth_grads, warn_shape, cu_seqlens)
-    mode = MODE_CAUSAL if is_causal else MODE_NONCAUSAL
-    o, lse = _ModaFunction.apply(q, k, v, cached_k, cached_v, scale, moda_group_num, mode)
+    o, lse = _attention(q, k, v, cached_k, cached_v, scale, moda_group_num, mode)
     return (o, lse) if need_lse else o
 
 
@@ -273,11 +214,16 @@ def parallel_moda_chunk_visible(q, k, v, g=None, cached_k=None, cached_v=None, s
                                 customized_BS_backward=None):
     """Causal MoDA whose queries also see the depth KV of earlier positions of their
     64-query-row chunk (reference: moda_v16.py:3614-3651; oracle chunk_size = 64 // G)."""
+    if g is None and cu_seqlens is None and not head_first:
+        r = _cabi.native().attention(q, k, v, cached_k, cached_v, scale, moda_group_num, MODE_CHUNK_VISIBLE,
+                                     return_depth_grads, warn_shape, False)
+        if r is not None:
+            return r if need_lse else r[0]
     assert CHUNK_VISIBLE_QUERY_ROWS % moda_group_num == 0, "moda_group_num must divide 64"
     q, k, v, cached_k, cached_v, scale = _prepare(
         "parallel_moda_chunk_visible", q, k, v, g, cached_k, cached_v, scale, moda_group_num,
         head_first, return_depth_grads, warn_shape, cu_seqlens)
-    o, lse = _ModaFunction.apply(q, k, v, cached_k, cached_v, scale, moda_group_num, MODE_CHUNK_VISIBLE)
+    o, lse = _attention(q, k, v, cached_k, cached_v, scale, moda_group_num, MODE_CHUNK_VISIBLE)
     return (o, lse) if need_lse else o
 
 
@@ -289,11 +235,16 @@ def parallel_fda(q, k=None, v=None, g=None, cached_k=None, cached_v=None, scale=
     """Flash depth attention: each query attends only to the L depth KV of its own
     position (reference: fda_v12.py:1346-1449)."""
     assert k is None and v is None, "Flash Depth Attention does not accept legacy k/v; pass None"
+    if g is None and cu_seqlens is None and not head_first:
+        r = _cabi.native().attention(q, None, None, cached_k, cached_v, scale, moda_group_num, MODE_DEPTH_ONLY,
+                                     return_depth_grads, warn_shape, False)
+        if r is not None:
+            return r if need_lse else r[0]
     q, _, _, cached_k, cached_v, scale = _prepare(
         "parallel_fda", q, None, None, g, cached_k, cached_v, scale, moda_group_num, head_first,
         return_depth_grads, warn_shape, cu_seqlens, need_kv=False)
     assert cached_k is not None, "Flash Depth Attention requires L >= 1"                # fda_v12.py:301
-    o, lse = _ModaFunction.apply(q, None, None, cached_k, cached_v, scale, moda_group_num, MODE_DEPTH_ONLY)
+    o, lse = _attention(q, None, None, cached_k, cached_v, scale, moda_group_num, MODE_DEPTH_ONLY)
     return (o, lse) if need_lse else o
 
 
