@@ -195,6 +195,14 @@ Params sequence_part(const Params& p) {
   s.merge_depth = 1;
   return s;
 }
+// The problem the attention kernels see: with the depth part split off it has no depth rows, so an
+// in-place cache of any layer count leaves the sequence part on the tcgen05 kernels.
+moda_problem attention_problem(const moda_problem* pr, bool is_bwd) {
+  moda_problem a = *pr;
+  if (split_depth(pr, is_bwd)) { a.L = 0; a.depth_rows_per_pos = 0; }
+  return a;
+}
+
 template <typename T, int D>
 int fda_fwd(const Params& p, int n_sm, cudaStream_t st) {
   const int64_t units = (int64_t)p.B * p.T_kv * p.H;
@@ -333,7 +341,8 @@ int moda_b200_fwd(const moda_problem* prob, const moda_tensor4* q, const moda_te
   if (int rc = check_tensor(depth_v, need_dep, prob->B, Td, prob->H)) return rc;
   if (int rc = check_tensor(o, true, prob->B, Tq, prob->H)) return rc;
   if (lse == nullptr) return MODA_ERR_NULL;
-  const int path = resolve_path(prob, false);
+  const moda_problem att = attention_problem(prob, false);
+  const int path = resolve_path(&att, false);
   if (path < 0) return -path;
 
   Params p{};
@@ -357,7 +366,7 @@ int moda_b200_fwd(const moda_problem* prob, const moda_tensor4* q, const moda_te
     p = sequence_part(p);
   }
 #ifndef MODA_NO_TCGEN05
-  if (path == MODA_PATH_TCGEN05) return tc_forward(p, prob, n_sm, st);
+  if (path == MODA_PATH_TCGEN05) return tc_forward(p, &att, n_sm, st);
 #endif
   return prob->dtype == MODA_BF16 ? simt_fwd_d<__nv_bfloat16>(p, prob->D, st)
                                   : simt_fwd_d<__half>(p, prob->D, st);
@@ -368,7 +377,8 @@ int moda_b200_bwd_workspace_bytes(const moda_problem* prob, size_t* bytes) {
   if (int rc = check_problem(prob)) return rc;
   size_t n = delta_bytes(prob);
 #ifndef MODA_NO_TCGEN05
-  n += tc::bwd_extra_workspace_bytes(prob);
+  const moda_problem att = attention_problem(prob, true);
+  n += tc::bwd_extra_workspace_bytes(&att);
 #endif
   *bytes = n;
   return MODA_OK;
@@ -403,7 +413,8 @@ int moda_b200_bwd(const moda_problem* prob, const moda_tensor4* q, const moda_te
   if (int rc = moda_b200_bwd_workspace_bytes(prob, &need)) return rc;
   if (workspace == nullptr || workspace_bytes < need) return MODA_ERR_WORKSPACE;
   if (reinterpret_cast<uintptr_t>(workspace) & 255u) return MODA_ERR_ALIGNMENT;
-  const int path = resolve_path(prob, true);
+  const moda_problem att = attention_problem(prob, true);
+  const int path = resolve_path(&att, true);
   if (path < 0) return -path;
 
   Params p{};
@@ -433,7 +444,7 @@ int moda_b200_bwd(const moda_problem* prob, const moda_tensor4* q, const moda_te
 #ifndef MODA_NO_TCGEN05
   if (path == MODA_PATH_TCGEN05) {
     void* extra = reinterpret_cast<unsigned char*>(workspace) + delta_bytes(prob);
-    return tc::bwd(p, prob, extra, n_sm, st, &g_last_launches, &g_last_cuda_error);
+    return tc::bwd(p, &att, extra, n_sm, st, &g_last_launches, &g_last_cuda_error);
   }
 #endif
   return prob->dtype == MODA_BF16 ? simt_bwd_d<__nv_bfloat16>(p, prob->D, n_sm, st)
