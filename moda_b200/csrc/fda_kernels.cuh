@@ -1,19 +1,52 @@
 // Depth-only attention (parallel_fda, fda_v12.py:1346) as HBM-bandwidth kernels.
 //
 // Each query position attends only to the L depth K/V rows of its own position, so the
-// operator moves 2*L*D elements per position for 4*G*L*D flops: about 1 flop per byte.  The
-// attention-tile pipeline (tensor cores, 128-row tiles) would multiply every query against
-// the depth rows of 127 other positions; here one warp owns one (batch, position, head),
-// streams its L K rows and L V rows once with 16-byte loads (8 lanes per 256-byte row, four
-// rows per pass, sixteen rows per online-softmax block), keeps scores, softmax and accumulators in fp32 registers, and writes o /
-// lse (forward) or dq, d_depth_k, d_depth_v (backward; rows are owner-exclusive, no atomics).
+// operator moves 2*L*D elements per position for 4*G*L*D flops: about G flops per byte.  The
+// attention-tile pipeline (128-row tiles) would multiply every query against the depth rows of 127
+// other positions; here one warp owns one (batch, position, head) - a unit - and writes o / lse
+// (forward) or dq, d_depth_k, d_depth_v (backward; rows are owner-exclusive, no atomics).
 // Numerics as in the other kernels: scores scaled by scale*log2(e), exp2, lse = m + log2(l),
 // delta from the stored o, dq and dk scaled by `scale` at the end.
+//
+// A unit's K/V rows are a few KB (11 rows of 128 bytes in a vision transformer), so two things
+// bound such a kernel before HBM does: the instructions of a unit, and the time between a unit's
+// loads and its last store.
+//  * Instructions: the up to 8 query rows of a position are columns of m16n8k16 matrix instructions.
+//    Per 16 depth rows that replaces 16 fp32 FMAs for every 16 bytes of K or V and query row, and
+//    the reductions over the lanes of a row.
+//  * Latency: every warp has two shared-memory stages of 16 K rows + 16 V rows (and the query rows of
+//    its units), so that the loads of the next step, usually another unit's, are under way while
+//    this one is computed.  TMA fills them: one lane, three to seven instructions a step and hardly
+//    any address arithmetic (filled by 16-byte cp.async, a unit of 11 rows of D = 64 took 740
+//    instructions, as many as on fp32 FMAs).  The backward's gradient rows take the place of the K
+//    and V rows of their stage and leave by TMA too.
+// Against the fp32-FMA kernels these replace: B = 256, T = 197, H = 6, D = 64, L = 11: forward 0.356 ->
+// 0.168 ms, backward 0.479 -> 0.298 ms (6.2 of the measured 6.56 TB/s copy bandwidth); D = 128, L = 32, G = 1 (53 GB):
+// 8.53 -> 7.90 ms; B = 2, T = 4093, H = 4, G = 4, D = 128, L = 24: 0.241 -> 0.085 ms and, against the
+// attention-tile mma.sync kernels, 0.520 -> 0.149 ms.
+//
+// Lane layout: g = lane >> 2, t = lane & 3.  A chunk is 16 bytes = 8 channels of a row.
+//  * K (and q, dO; V for dO V^T): lane (g, t) takes chunks t, t + 4, .. of row g.  Word w of chunk
+//    t + 4 j is the operand of k-step (j, w >> 1): the channels a k-step contracts are permuted the
+//    same way in both operands, which a sum does not see.
+//  * V (for P V; K for dS K): lane (g, t) takes chunks g, g + 8, .. of four rows; byte permutations of
+//    two of them make the operand of a channel with the depth rows as the contracted index.
+//  * An 8 x 8 transpose (movmatrix) of the words of the first layout gives the right operand with
+//    the query rows as the contracted index, for channels 32 j + 8 t + 2 w, + 1 of the result: a lane's
+//    results of the four words are one 16-byte chunk.
+// P and dS enter as two 16-bit numbers each, the value and what its rounding left over (2^-17 relative
+// for bf16), not as one: the probabilities keep the precision they have as fp32 numbers next to
+// 16-bit K, V and results.
 #pragma once
 #include "common.cuh"
+#include "simt_mma_kernels.cuh"
+#include "tc_bwd_kernels.cuh"
 
 namespace moda {
 namespace fda {
+
+constexpr int kWarps = 4;             // warps of a block: they share nothing but the launch
+constexpr int kRows = 16;             // depth rows of a stage
 
 template <typename T> __device__ __forceinline__ void unpack8(const uint4& u, float (&f)[8]) {
   const float2 a = Pack<T>::unpack(u.x), b = Pack<T>::unpack(u.y), c = Pack<T>::unpack(u.z), d = Pack<T>::unpack(u.w);
@@ -29,278 +62,491 @@ template <typename T> __device__ __forceinline__ void add8(float (&f)[8], const 
 template <typename T> __device__ __forceinline__ uint4 pack8(const float (&f)[8]) {
   return make_uint4(Pack<T>::pack(f[0], f[1]), Pack<T>::pack(f[2], f[3]), Pack<T>::pack(f[4], f[5]), Pack<T>::pack(f[6], f[7]));
 }
-__device__ __forceinline__ float group8_sum(float x) {   // sum over the 8 lanes that share a row
+__device__ __forceinline__ uint32_t transpose8x8(uint32_t x) {
+  uint32_t y;
+  asm volatile("movmatrix.sync.aligned.m8n8.trans.b16 %0, %1;" : "=r"(y) : "r"(x));
+  return y;
+}
+// (a, b) as a 16-bit pair and the pair of what the rounding left over
+template <typename T> __device__ __forceinline__ void split_pair(float a, float b, uint32_t& hi, uint32_t& lo) {
+  hi = Pack<T>::pack(a, b);
+  const float2 h = Pack<T>::unpack(hi);
+  lo = Pack<T>::pack(a - h.x, b - h.y);
+}
+__device__ __forceinline__ float quad_sum(float x) {
   x += __shfl_xor_sync(0xffffffffu, x, 1);
-  x += __shfl_xor_sync(0xffffffffu, x, 2);
-  x += __shfl_xor_sync(0xffffffffu, x, 4);
-  return x;
-}
-__device__ __forceinline__ float cross4_sum(float x) {   // sum over the 4 row groups of a warp
-  x += __shfl_xor_sync(0xffffffffu, x, 8);
-  x += __shfl_xor_sync(0xffffffffu, x, 16);
-  return x;
-}
-__device__ __forceinline__ float cross4_max(float x) {
-  x = fmaxf(x, __shfl_xor_sync(0xffffffffu, x, 8));
-  x = fmaxf(x, __shfl_xor_sync(0xffffffffu, x, 16));
-  return x;
+  return x + __shfl_xor_sync(0xffffffffu, x, 2);
 }
 
-// (b, t, h) of a flattened unit index; 32-bit division when the index fits (64-bit division
-// costs hundreds of clocks, which a unit with a few KB of depth rows does not hide).
-__device__ __forceinline__ void decode_unit(int64_t unit, int H, int T_kv, int& b, int& t, int& h) {
-  if (unit <= 0x7fffffffLL) {
-    const unsigned u = (unsigned)unit, uh = u / (unsigned)H;
-    h = (int)(u - uh * (unsigned)H);
-    b = (int)(uh / (unsigned)T_kv);
-    t = (int)(uh - (unsigned)b * (unsigned)T_kv);
-  } else {
-    h = (int)(unit % H);
-    t = (int)((unit / H) % T_kv);
-    b = (int)(unit / ((int64_t)H * T_kv));
+// Rows of a stage are permuted so that both ways of reading it are free of bank conflicts under the
+// TMA unit's 128-byte swizzle (chunk c of row r sits at chunk c ^ (r & 7)): column 2 t + e of matrix
+// operand nt is tile row 8 nt + row_of(t, e).  Two lanes of a K access then differ in bit 2 of the row,
+// the four rows of a V access (same e) in bits 1 and 2.
+__device__ __forceinline__ int row_of(int t, int e) {
+  // t: 0 1 2 3 -> e = 0: 0 2 5 7, e = 1: 4 6 1 3
+  return (2 * t + (t >> 1)) ^ (e << 2);
+}
+// 16-byte chunk c of row r of a tile of 64-channel boxes of `rows` rows each
+template <int ROWS> __device__ __forceinline__ uint32_t chunk_at(int r, int c) { return (c >> 3) * (ROWS * 128) + r * 128 + (((c & 7) ^ (r & 7)) << 4); }
+template <int ROWS> __device__ __forceinline__ uint4 tile_chunk(const unsigned char* tile, int r, int c) {
+  return *reinterpret_cast<const uint4*>(tile + chunk_at<ROWS>(r, c));
+}
+
+// One step of a warp: a block of 16 depth rows of a unit, for query rows [g0, g0 + 8) of its position.
+// Units are numbered h-fastest; a warp takes every (warps of the grid)-th one, and the step from one to
+// the next is an addition with carries (a division costs more than the rest of the bookkeeping).
+struct Step { int b, t, h, l0, g0; };
+struct Stride {
+  int b, t, h;
+  __device__ __forceinline__ Stride(const Params& p, unsigned n) {
+    h = (int)(n % (unsigned)p.H);
+    n /= (unsigned)p.H;
+    t = (int)(n % (unsigned)p.T_kv);
+    b = (int)(n / (unsigned)p.T_kv);
   }
+  __device__ __forceinline__ void advance(const Params& p, Step& s) const {
+    s.l0 += kRows;
+    if (s.l0 < p.L) return;
+    s.l0 = 0;
+    s.g0 += 8;
+    if (s.g0 < p.G) return;
+    s.g0 = 0;
+    s.h += h;
+    if (s.h >= p.H) { s.h -= p.H; ++s.t; }
+    s.t += t;
+    if (s.t >= p.T_kv) { s.t -= p.T_kv; ++s.b; }
+    s.b += b;
+  }
+};
+
+__device__ __forceinline__ Step first_step(const Params& p) {
+  const Stride at(p, blockIdx.x * kWarps + (threadIdx.x >> 5));
+  return Step{at.b, at.t, at.h, 0, 0};
 }
 
-// Lane layout: sub = lane & 7 picks the 16-byte chunks {sub, sub + 8, ...} of a row (CH = D/64
-// chunks per lane), grp = lane >> 3 picks which of the 4 rows of a pass the lane works on.
+// k, v: boxes of 16 depth rows x 64 channels; kt, vt: of the L % 16 rows of a unit's last block, so that
+// nothing of the next position (or of a cache's unwritten layers) is read.  q, dout, o: the query
+// rows of a position (8 of them at most), unswizzled.
+struct Maps { CUtensorMap k, v, kt, vt, q, dout, o; };
+struct OutMaps { CUtensorMap dk, dv, dkt, dvt; };     // the same boxes of the depth gradients
 
-// ------------------------------------------------------------------------- forward
-// One warp per (b, t, h); all G query rows of the position reuse the K/V rows (L1-resident on
-// the second and later reads).  With 128-byte rows (D = 64) a unit is a few KB and the kernels are
-// bound by latency and instruction issue rather than by HBM, so more warps are kept resident there.
-template <typename T, int D>
-__global__ void __launch_bounds__(256, D == 64 ? 3 : 2) fwd_kernel(const __grid_constant__ Params p) {
-  constexpr int CH = D / 64;
-  const int lane = threadIdx.x & 31, sub = lane & 7, grp = lane >> 3;
-  const int64_t n_units = (int64_t)p.B * p.T_kv * p.H;
-  const int64_t wstride = (int64_t)gridDim.x * (blockDim.x >> 5);
-  for (int64_t unit = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); unit < n_units; unit += wstride) {
-    int b, t, h;
-    decode_unit(unit, p.H, p.T_kv, b, t, h);
-    const T* kb = reinterpret_cast<const T*>(p.kd.ptr) + p.kd.off(b, (int64_t)t * p.Ls, h);
-    const T* vb = reinterpret_cast<const T*>(p.vd.ptr) + p.vd.off(b, (int64_t)t * p.Ls, h);
-    for (int g = 0; g < p.G; ++g) {
-      const int r = t * p.G + g;
-      float qf[CH][8];
-      {
-        const T* qp = reinterpret_cast<const T*>(p.q.ptr) + p.q.off(b, r, h);
-#pragma unroll
-        for (int c = 0; c < CH; ++c) {
-          unpack8<T>(*reinterpret_cast<const uint4*>(qp + (sub + 8 * c) * 8), qf[c]);
-#pragma unroll
-          for (int e = 0; e < 8; ++e) qf[c][e] *= p.scale_log2;
-        }
-      }
-      float m = -INFINITY, lsum = 0.f;
-      float acc[CH][8];
-#pragma unroll
-      for (int c = 0; c < CH; ++c)
-#pragma unroll
-        for (int e = 0; e < 8; ++e) acc[c][e] = 0.f;
+// Shared memory of a block: per warp two stages {K tile, V tile}; per warp one group of the query rows
+// of q (NQ = 1) or q, dout, o (NQ = 3); per warp two mbarriers; the abort words.
+template <int D> __host__ __device__ constexpr uint32_t tile_bytes() { return kRows * 2 * D; }
+template <int D, int NQ> __host__ __device__ constexpr uint32_t smem_bytes(int G) {
+  return kWarps * (4 * tile_bytes<D>() + NQ * (G < 8 ? G : 8) * 2 * D + 16) + 16;
+}
 
-      for (int l0 = 0; l0 < p.L; l0 += 16) {
-        uint4 raw[4][CH];
-        uint4 vraw[4][1];                         // D = 64: the V rows travel with the K rows
-        float s[4];
-#pragma unroll
-        for (int ps = 0; ps < 4; ++ps) {          // all K loads of the block in flight together
-          const int key = l0 + ps * 4 + grp;
-#pragma unroll
-          for (int c = 0; c < CH; ++c)
-            raw[ps][c] = (key < p.L) ? *reinterpret_cast<const uint4*>(kb + (int64_t)key * p.kd.st + (sub + 8 * c) * 8)
-                                     : make_uint4(0, 0, 0, 0);
-          if constexpr (CH == 1)
-            vraw[ps][0] = (key < p.L) ? *reinterpret_cast<const uint4*>(vb + (int64_t)key * p.vd.st + sub * 8)
-                                      : make_uint4(0, 0, 0, 0);
+// The ring of one warp.
+template <int D, int NQ>
+struct Ring {
+  unsigned char *tiles, *queries;
+  uint32_t bars;
+  volatile int* abort_flag;
+  int issued = 0, taken = 0;           // steps issued / taken so far
+  __device__ __forceinline__ Ring(const Params& p, unsigned char* smem) {
+    const int w = threadIdx.x >> 5;
+    const uint32_t q_bytes = NQ * min(p.G, 8) * 2 * D;
+    tiles = smem + w * 4 * tile_bytes<D>();
+    queries = smem + kWarps * 4 * tile_bytes<D>() + w * q_bytes;
+    unsigned char* ctl = smem + kWarps * (4 * tile_bytes<D>() + q_bytes);
+    bars = smem_u32(ctl) + w * 16;
+    abort_flag = reinterpret_cast<volatile int*>(ctl + kWarps * 16);     // {abort, call}, {drain, call}
+    if (threadIdx.x == 0) { tc::arm_abort(abort_flag, p); tc::arm_abort(abort_flag + 2, p); }
+    if ((threadIdx.x & 31) == 0) {
+      tc::mbar_init(bars, 1);
+      tc::mbar_init(bars + 8, 1);
+      asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    }
+    __syncthreads();
+  }
+  // Loads of step s; a unit's first step brings the query rows.
+  __device__ __forceinline__ void issue(const Params& p, const Maps& maps, const Step& s) {
+    if (tc::elect_one()) {
+      const int n = min(p.L - s.l0, kRows), row = s.t * p.Ls + s.l0;
+      const uint32_t bar = bars + 8 * (issued & 1), dst = smem_u32(tiles) + (issued & 1) * 2 * tile_bytes<D>();
+      const uint32_t q_rows = min(p.G, 8) * 2 * D;
+      tc::mbar_expect_tx(bar, n * 4 * D + (s.l0 == 0 ? NQ * q_rows : 0));
+      tc::tma_load_tile<D>(dst, n == kRows ? &maps.k : &maps.kt, bar, kRows * 128, s.h, row, s.b);
+      tc::tma_load_tile<D>(dst + tile_bytes<D>(), n == kRows ? &maps.v : &maps.vt, bar, kRows * 128, s.h, row, s.b);
+      if (s.l0 == 0) {
+        const int r = s.t * p.G + s.g0;
+        tc::tma_load_4d(smem_u32(queries), &maps.q, bar, 0, s.h, r, s.b);
+        if constexpr (NQ == 3) {
+          tc::tma_load_4d(smem_u32(queries) + q_rows, &maps.dout, bar, 0, s.h, r, s.b);
+          tc::tma_load_4d(smem_u32(queries) + 2 * q_rows, &maps.o, bar, 0, s.h, r, s.b);
         }
-        float bm = -INFINITY;
-#pragma unroll
-        for (int ps = 0; ps < 4; ++ps) {
-          float d = 0.f;
-#pragma unroll
-          for (int c = 0; c < CH; ++c) {
-            float kf[8];
-            unpack8<T>(raw[ps][c], kf);
-#pragma unroll
-            for (int e = 0; e < 8; ++e) d = fmaf(qf[c][e], kf[e], d);
-          }
-          d = group8_sum(d);
-          s[ps] = (l0 + ps * 4 + grp < p.L) ? d : -INFINITY;
-          bm = fmaxf(bm, s[ps]);
-        }
-        bm = cross4_max(bm);
-        const float m_new = fmaxf(m, bm);          // finite: key l0 of the block is always valid
-        const float alpha = fast_exp2(m - m_new);
-        m = m_new;
-        lsum *= alpha;
-#pragma unroll
-        for (int c = 0; c < CH; ++c)
-#pragma unroll
-          for (int e = 0; e < 8; ++e) acc[c][e] *= alpha;
-        if constexpr (CH == 1) {
-#pragma unroll
-          for (int ps = 0; ps < 4; ++ps) raw[ps][0] = vraw[ps][0];
-        } else {
-#pragma unroll
-          for (int ps = 0; ps < 4; ++ps) {          // V loads of the block
-            const int key = l0 + ps * 4 + grp;
-#pragma unroll
-            for (int c = 0; c < CH; ++c)
-              raw[ps][c] = (key < p.L) ? *reinterpret_cast<const uint4*>(vb + (int64_t)key * p.vd.st + (sub + 8 * c) * 8)
-                                       : make_uint4(0, 0, 0, 0);
-          }
-        }
-#pragma unroll
-        for (int ps = 0; ps < 4; ++ps) {
-          const float pw = fast_exp2(s[ps] - m);  // 0 for invalid keys (s = -inf)
-          lsum += pw;
-#pragma unroll
-          for (int c = 0; c < CH; ++c) {
-            float vf[8];
-            unpack8<T>(raw[ps][c], vf);
-#pragma unroll
-            for (int e = 0; e < 8; ++e) acc[c][e] = fmaf(pw, vf[e], acc[c][e]);
-          }
-        }
-      }
-      lsum = cross4_sum(lsum);
-      const float inv = 1.f / lsum;
-#pragma unroll
-      for (int c = 0; c < CH; ++c)
-#pragma unroll
-        for (int e = 0; e < 8; ++e) acc[c][e] = cross4_sum(acc[c][e]) * inv;
-      if (grp == 0) {
-        T* op = reinterpret_cast<T*>(p.o.ptr) + p.o.off(b, r, h);
-#pragma unroll
-        for (int c = 0; c < CH; ++c) *reinterpret_cast<uint4*>(op + (sub + 8 * c) * 8) = pack8<T>(acc[c]);
-        if (sub == 0) p.lse[((int64_t)b * p.T_q + r) * p.H + h] = m + log2f(lsum);
       }
     }
+    __syncwarp();
+    ++issued;
   }
+  // Waits for the next step's rows; false: the wait expired (bounded, as everywhere).
+  __device__ __forceinline__ bool wait() {
+    const bool ok = __all_sync(0xffffffffu, tc::mbar_wait(bars + 8 * (taken & 1), (taken >> 1) & 1, abort_flag, 30));
+    ++taken;
+    return ok;
+  }
+  // The stage of the current step, which now holds gradient rows, to memory; the lane that stores is the
+  // one that waits (stored_read) before the stage is filled again.
+  __device__ __forceinline__ void store(const Params& p, const OutMaps& maps, const Step& s) {
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    __syncwarp();
+    if (tc::elect_one()) {
+      const bool full = p.L - s.l0 >= kRows;
+      const uint32_t src = smem_u32(tiles) + ((taken - 1) & 1) * 2 * tile_bytes<D>();
+      const int row = s.t * p.Ls + s.l0;
+#pragma unroll
+      for (int bx = 0; bx < D / 64; ++bx) {
+        tc::tma_store_4d(full ? &maps.dk : &maps.dkt, src + bx * kRows * 128, 64 * bx, s.h, row, s.b);
+        tc::tma_store_4d(full ? &maps.dv : &maps.dvt, src + tile_bytes<D>() + bx * kRows * 128, 64 * bx, s.h, row, s.b);
+      }
+      tc::bulk_commit();
+    }
+    __syncwarp();
+  }
+  __device__ __forceinline__ void stored_read() {
+    if (tc::elect_one()) tc::bulk_wait_read_all();
+    __syncwarp();
+  }
+  // After a failed wait: loads in flight land before the shared memory is given up.
+  __device__ __forceinline__ void drain() {
+    for (int i = taken - 1; i < issued; ++i) tc::mbar_wait(bars + 8 * (i & 1), (i >> 1) & 1, abort_flag + 2, 30);
+  }
+  __device__ __forceinline__ const unsigned char* stage() const { return tiles + ((taken - 1) & 1) * 2 * tile_bytes<D>(); }
+};
+template <int D> __device__ __forceinline__ uint4 query_chunk(const unsigned char* rows, int r, int c) {
+  return *reinterpret_cast<const uint4*>(rows + r * 2 * D + c * 16);
+}
+
+// acc[i] += (rows of `tile`)^T x: for 64 channels of a tile (box i) the 8 channels of chunk g as left
+// operands, each made from the tile rows of operand columns 2 t, 2 t + 1 (+ 8), and the pair x of
+// right operands (16-bit values and what their rounding left over).  Result [e][c]: channel 8 g + e
+// of query 2 t + c.  `left` rows of the tile exist (kAll: all, or the others are zeros).
+template <typename T, bool kAll>
+__device__ __forceinline__ void add_transposed(float (&acc)[8][2], const unsigned char* tile, int i, int g, int t4, int left,
+                                               const uint32_t (&hi)[2], const uint32_t (&lo)[2]) {
+  uint32_t w[4][4];
+#pragma unroll
+  for (int x = 0; x < 4; ++x) {                     // a row that does not exist is whatever the stage held before
+    const int r = 8 * (x >> 1) + row_of(t4, x & 1);
+    const uint4 v4 = kAll || r < left ? tile_chunk<kRows>(tile, r, g + 8 * i) : make_uint4(0, 0, 0, 0);
+    w[x][0] = v4.x; w[x][1] = v4.y; w[x][2] = v4.z; w[x][3] = v4.w;
+  }
+#pragma unroll
+  for (int e = 0; e < 4; ++e) {                     // channels 2 e (rows g of the operand) and 2 e + 1 (rows g + 8)
+    const uint32_t a[4] = {__byte_perm(w[0][e], w[1][e], 0x5410u), __byte_perm(w[0][e], w[1][e], 0x7632u),
+                           __byte_perm(w[2][e], w[3][e], 0x5410u), __byte_perm(w[2][e], w[3][e], 0x7632u)};
+    float c[4] = {acc[2 * e][0], acc[2 * e][1], acc[2 * e + 1][0], acc[2 * e + 1][1]};
+    simt::Mma<T>::run(c, a, hi[0], hi[1]);
+    simt::Mma<T>::run(c, a, lo[0], lo[1]);
+    acc[2 * e][0] = c[0]; acc[2 * e][1] = c[1]; acc[2 * e + 1][0] = c[2]; acc[2 * e + 1][1] = c[3];
+  }
+}
+
+// kOne: L <= 16, a unit is one step.  The rows of a stage that no unit fills are then zeroed once, the
+// probabilities are normalised before P V, and nothing is carried from step to step.
+template <int D, int NQ> __device__ __forceinline__ void zero_tiles(const Ring<D, NQ>& ring) {
+  for (uint32_t i = (threadIdx.x & 31) * 16; i < 4 * tile_bytes<D>(); i += 32 * 16) *reinterpret_cast<uint4*>(ring.tiles + i) = make_uint4(0, 0, 0, 0);
+  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");     // before the TMA unit writes there
+  __syncwarp();
+}
+
+// ------------------------------------------------------------------------- forward
+template <typename T, int D, bool kOne>
+__global__ void __launch_bounds__(kWarps * 32, D == 64 ? 6 : 3) fwd_kernel(const __grid_constant__ Params p, const __grid_constant__ Maps maps) {
+  constexpr int J = D / 32, I = D / 64;
+  extern __shared__ __align__(1024) unsigned char smem[];
+  if (smem_u32(smem) & 1023u) {                     // the swizzle is a function of the shared-memory address
+    if (threadIdx.x == 0) tc::record_failure(2 << 8, p.launch_id);
+    return;
+  }
+  if (tc::launch_failed(p)) return;
+  const int lane = threadIdx.x & 31, g = lane >> 2, t4 = lane & 3;
+  const int my_row = row_of(g >> 1, g & 1);         // tile row (+ 8 nt) of this lane's K operand
+  Ring<D, 1> ring(p, smem);
+  if (kOne) zero_tiles(ring);
+  const Stride stride(p, gridDim.x * kWarps);
+  Step s = first_step(p);
+  if (s.b < p.B) ring.issue(p, maps, s);
+  uint4 qa[J];
+  float m = -INFINITY, lsum = 0.f;
+  float acc[I][8][2];                               // [channel 8 (g + 8 i) + e][query 2 t + c]
+  bool ok = true;
+  while (s.b < p.B) {
+    Step next = s;
+    stride.advance(p, next);
+    if (!(ok = ring.wait())) break;
+    const int n_rows = p.G - s.g0;                  // query rows of the step (8 or more: 8)
+    const bool first = kOne || s.l0 == 0;
+    if (first) {
+#pragma unroll
+      for (int j = 0; j < J; ++j) qa[j] = g < n_rows ? query_chunk<D>(ring.queries, g, t4 + 4 * j) : make_uint4(0, 0, 0, 0);
+    }
+    __syncwarp();                                   // the other stage and the query rows have been read
+    if (next.b < p.B) ring.issue(p, maps, next);
+    const unsigned char *kt = ring.stage(), *vt = kt + tile_bytes<D>();
+    const int left = p.L - s.l0;                    // rows of the tile that exist (16 or more: all)
+
+    float pv[4];                                    // scores of query g; columns 2 t, 2 t + 1, 8 + 2 t, 8 + 2 t + 1
+#pragma unroll
+    for (int nt = 0; nt < 2; ++nt) {
+      float sc[4] = {0.f, 0.f, 0.f, 0.f};           // [2], [3] stay 0
+#pragma unroll
+      for (int j = 0; j < J; ++j) {
+        const uint4 kw = tile_chunk<kRows>(kt, 8 * nt + my_row, t4 + 4 * j);
+        const uint32_t a0[4] = {qa[j].x, 0u, qa[j].y, 0u}, a1[4] = {qa[j].z, 0u, qa[j].w, 0u};
+        simt::Mma<T>::run(sc, a0, kw.x, kw.y);
+        simt::Mma<T>::run(sc, a1, kw.z, kw.w);
+      }
+      pv[2 * nt] = sc[0];
+      pv[2 * nt + 1] = sc[1];
+    }
+    float bm = -INFINITY;
+#pragma unroll
+    for (int x = 0; x < 4; ++x) {
+      pv[x] = 8 * (x >> 1) + row_of(t4, x & 1) < left ? pv[x] * p.scale_log2 : -INFINITY;
+      bm = fmaxf(bm, pv[x]);
+    }
+    bm = fmaxf(bm, __shfl_xor_sync(0xffffffffu, bm, 1));
+    bm = fmaxf(bm, __shfl_xor_sync(0xffffffffu, bm, 2));
+    const float m_old = m;
+    m = first ? bm : fmaxf(m, bm);                  // finite: the first row of a block always exists
+#pragma unroll
+    for (int x = 0; x < 4; ++x) pv[x] = fast_exp2(pv[x] - m);      // 0 for rows that do not exist
+    const float part = (pv[0] + pv[1]) + (pv[2] + pv[3]);
+    float total = 0.f;
+    if (kOne) {
+      total = quad_sum(part);
+      const float inv = 1.f / total;
+#pragma unroll
+      for (int x = 0; x < 4; ++x) pv[x] *= inv;
+    }
+    if (first) {
+      lsum = part;
+#pragma unroll
+      for (int i = 0; i < I; ++i)
+#pragma unroll
+        for (int e = 0; e < 8; ++e) acc[i][e][0] = acc[i][e][1] = 0.f;
+    } else {
+      const float alpha = fast_exp2(m_old - m);
+      lsum = fmaf(lsum, alpha, part);
+      const float a0 = __shfl_sync(0xffffffffu, alpha, 8 * t4), a1 = __shfl_sync(0xffffffffu, alpha, 8 * t4 + 4);   // queries 2 t, 2 t + 1
+#pragma unroll
+      for (int i = 0; i < I; ++i)
+#pragma unroll
+        for (int e = 0; e < 8; ++e) { acc[i][e][0] *= a0; acc[i][e][1] *= a1; }
+    }
+    uint32_t ph[2], pl[2];
+    split_pair<T>(pv[0], pv[1], ph[0], pl[0]);
+    split_pair<T>(pv[2], pv[3], ph[1], pl[1]);
+#pragma unroll
+    for (int i = 0; i < I; ++i) add_transposed<T, kOne>(acc[i], vt, i, g, t4, left, ph, pl);
+
+    if (kOne || left <= kRows) {
+      const int r = s.t * p.G + s.g0;
+      float inv[2] = {1.f, 1.f};
+      if (!kOne) {
+        total = quad_sum(lsum);
+        const float v = 1.f / total;
+        inv[0] = __shfl_sync(0xffffffffu, v, 8 * t4);
+        inv[1] = __shfl_sync(0xffffffffu, v, 8 * t4 + 4);
+      }
+      T* op = reinterpret_cast<T*>(p.o.ptr) + p.o.off(s.b, r + 2 * t4, s.h) + 8 * g;
+#pragma unroll
+      for (int c = 0; c < 2; ++c)
+        if (2 * t4 + c < n_rows)
+#pragma unroll
+          for (int i = 0; i < I; ++i) {
+            float f[8];
+#pragma unroll
+            for (int e = 0; e < 8; ++e) f[e] = kOne ? acc[i][e][c] : acc[i][e][c] * inv[c];
+            *reinterpret_cast<uint4*>(op + c * p.o.st + 64 * i) = pack8<T>(f);
+          }
+      if (t4 == 0 && g < n_rows) p.lse[((int64_t)s.b * p.T_q + r + g) * p.H + s.h] = m + log2f(total);
+    }
+    s = next;
+  }
+  if (!ok) ring.drain();
 }
 
 // ------------------------------------------------------------------------- backward
-// One warp per (b, t, h), G query rows held in registers (G is a template parameter).
-template <typename T, int D, int G>
-__global__ void __launch_bounds__(128, (G == 1) ? (D == 64 ? 5 : 3) : 2) bwd_kernel(const __grid_constant__ Params p) {
-  constexpr int CH = D / 64;
-  const int lane = threadIdx.x & 31, sub = lane & 7, grp = lane >> 3;
-  const int64_t n_units = (int64_t)p.B * p.T_kv * p.H;
-  const int64_t wstride = (int64_t)gridDim.x * (blockDim.x >> 5);
-  for (int64_t unit = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); unit < n_units; unit += wstride) {
-    int b, t, h;
-    decode_unit(unit, p.H, p.T_kv, b, t, h);
-    const T* kb = reinterpret_cast<const T*>(p.kd.ptr) + p.kd.off(b, (int64_t)t * p.Ls, h);
-    const T* vb = reinterpret_cast<const T*>(p.vd.ptr) + p.vd.off(b, (int64_t)t * p.Ls, h);
-    T* dkb = reinterpret_cast<T*>(p.dkd.ptr) + p.dkd.off(b, (int64_t)t * p.Ls, h);
-    T* dvb = reinterpret_cast<T*>(p.dvd.ptr) + p.dvd.off(b, (int64_t)t * p.Ls, h);
-
-    uint4 qraw[G][CH], doraw[G][CH];
-    float lse_g[G], delta_g[G];
-    float dq[G][CH][8];
+// G <= 8: the query rows of a position are one group.  Scores are computed transposed (K as the left
+// operand: 16 depth rows at once), so that P^T and dS^T are left operands of dV = P^T dO and
+// dK = dS^T Q as they come.
+template <typename T, int D, bool kOne, bool kAdd>
+__global__ void __launch_bounds__(kWarps * 32, D == 64 ? (kOne ? 5 : 4) : 3) bwd_kernel(const __grid_constant__ Params p, const __grid_constant__ Maps maps, const __grid_constant__ OutMaps omaps) {
+  constexpr int J = D / 32, I = D / 64;
+  extern __shared__ __align__(1024) unsigned char smem[];
+  if (smem_u32(smem) & 1023u) {
+    if (threadIdx.x == 0) tc::record_failure(2 << 8, p.launch_id);
+    return;
+  }
+  if (tc::launch_failed(p)) return;
+  const int lane = threadIdx.x & 31, g = lane >> 2, t4 = lane & 3;
+  const int my_row = row_of(g >> 1, g & 1);         // tile row (+ 8) of this lane's operands and results
+  const bool row_ok = g < p.G;
+  Ring<D, 3> ring(p, smem);
+  if (kOne) zero_tiles(ring);
+  const Stride stride(p, gridDim.x * kWarps);
+  Step s = first_step(p);
+  uint4 qa[J], da[J];
+  float delta[2] = {0.f, 0.f}, lse[2] = {0.f, 0.f};          // of queries 2 t, 2 t + 1
+  float lse_next[2] = {INFINITY, INFINITY};                  // P of a query that does not exist: exp2(-inf) = 0
+  float dq[I][8][2];                                         // [channel 8 (g + 8 i) + e][query 2 t + c]
+  bool ok = true;
+  auto issue = [&](const Step& x) {
+    ring.issue(p, maps, x);
+    if (kOne || x.l0 == 0) {
+      const float* l = p.lse + ((int64_t)x.b * p.T_q + x.t * p.G + 2 * t4) * p.H + x.h;
 #pragma unroll
-    for (int g = 0; g < G; ++g) {
-      const int r = t * G + g;
-      const T* qp = reinterpret_cast<const T*>(p.q.ptr) + p.q.off(b, r, h);
-      const T* dp_ = reinterpret_cast<const T*>(p.dout.ptr) + p.dout.off(b, r, h);
-      const T* op = reinterpret_cast<const T*>(p.o.ptr) + p.o.off(b, r, h);
+      for (int c = 0; c < 2; ++c)
+        if (2 * t4 + c < p.G) lse_next[c] = l[c * p.H];
+    }
+  };
+  if (s.b < p.B) issue(s);
+  while (s.b < p.B) {
+    Step next = s;
+    stride.advance(p, next);
+    if (!(ok = ring.wait())) break;
+    if (kOne || s.l0 == 0) {
+      lse[0] = lse_next[0];
+      lse[1] = lse_next[1];
       float dl = 0.f;
 #pragma unroll
-      for (int c = 0; c < CH; ++c) {
-        qraw[g][c] = *reinterpret_cast<const uint4*>(qp + (sub + 8 * c) * 8);
-        doraw[g][c] = *reinterpret_cast<const uint4*>(dp_ + (sub + 8 * c) * 8);
+      for (int j = 0; j < J; ++j) {
+        const uint4 zero = make_uint4(0, 0, 0, 0);
+        qa[j] = row_ok ? query_chunk<D>(ring.queries, g, t4 + 4 * j) : zero;
+        da[j] = row_ok ? query_chunk<D>(ring.queries + p.G * 2 * D, g, t4 + 4 * j) : zero;
+        const uint4 oa = row_ok ? query_chunk<D>(ring.queries + 2 * p.G * 2 * D, g, t4 + 4 * j) : zero;
         float of[8], df[8];
-        unpack8<T>(*reinterpret_cast<const uint4*>(op + (sub + 8 * c) * 8), of);
-        unpack8<T>(doraw[g][c], df);
+        unpack8<T>(oa, of);
+        unpack8<T>(da[j], df);
 #pragma unroll
-        for (int e = 0; e < 8; ++e) { dl = fmaf(of[e], df[e], dl); dq[g][c][e] = 0.f; }
+        for (int e = 0; e < 8; ++e) dl = fmaf(of[e], df[e], dl);
       }
-      delta_g[g] = group8_sum(dl);
-      lse_g[g] = p.lse[((int64_t)b * p.T_q + r) * p.H + h];
+      dl = quad_sum(dl);
+      delta[0] = __shfl_sync(0xffffffffu, dl, 8 * t4);
+      delta[1] = __shfl_sync(0xffffffffu, dl, 8 * t4 + 4);
+#pragma unroll
+      for (int i = 0; i < I; ++i)
+#pragma unroll
+        for (int e = 0; e < 8; ++e) dq[i][e][0] = dq[i][e][1] = 0.f;
     }
+    ring.stored_read();                             // the other stage and the query rows have been read
+    if (next.b < p.B) issue(next);
+    const unsigned char *kt = ring.stage(), *vt = kt + tile_bytes<D>();
+    const int left = p.L - s.l0;                    // rows of the tile that exist (16 or more: all)
 
-    for (int l0 = 0; l0 < p.L; l0 += 16) {
-      uint4 kraw[4][CH], vraw[4][CH];
+    // S^T and dP^T: [2 nt + c] = (tile row my_row + 8 nt, query 2 t + c)
+    float sc[4] = {0.f, 0.f, 0.f, 0.f}, dp[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
-      for (int ps = 0; ps < 4; ++ps) {
-        const int key = l0 + ps * 4 + grp;
-#pragma unroll
-        for (int c = 0; c < CH; ++c) {
-          const bool valid = key < p.L;
-          kraw[ps][c] = valid ? *reinterpret_cast<const uint4*>(kb + (int64_t)key * p.kd.st + (sub + 8 * c) * 8) : make_uint4(0, 0, 0, 0);
-          vraw[ps][c] = valid ? *reinterpret_cast<const uint4*>(vb + (int64_t)key * p.vd.st + (sub + 8 * c) * 8) : make_uint4(0, 0, 0, 0);
-        }
-      }
-#pragma unroll
-      for (int ps = 0; ps < 4; ++ps) {
-        const int key = l0 + ps * 4 + grp;
-        const bool valid = key < p.L;
-        float kf[CH][8], vf[CH][8], dkr[CH][8], dvr[CH][8];
-#pragma unroll
-        for (int c = 0; c < CH; ++c) {
-          unpack8<T>(kraw[ps][c], kf[c]);
-          unpack8<T>(vraw[ps][c], vf[c]);
-#pragma unroll
-          for (int e = 0; e < 8; ++e) { dkr[c][e] = 0.f; dvr[c][e] = 0.f; }
-        }
-#pragma unroll
-        for (int g = 0; g < G; ++g) {
-          float s = 0.f, dpv = 0.f;
-          float qf[CH][8], df[CH][8];
-#pragma unroll
-          for (int c = 0; c < CH; ++c) {
-            unpack8<T>(qraw[g][c], qf[c]);
-            unpack8<T>(doraw[g][c], df[c]);
-#pragma unroll
-            for (int e = 0; e < 8; ++e) { s = fmaf(qf[c][e], kf[c][e], s); dpv = fmaf(df[c][e], vf[c][e], dpv); }
-          }
-          s = group8_sum(s);
-          dpv = group8_sum(dpv);
-          const float pw = valid ? fast_exp2(fmaf(s, p.scale_log2, -lse_g[g])) : 0.f;
-          const float ds = pw * (dpv - delta_g[g]);
-#pragma unroll
-          for (int c = 0; c < CH; ++c)
-#pragma unroll
-            for (int e = 0; e < 8; ++e) {
-              dq[g][c][e] = fmaf(ds, kf[c][e], dq[g][c][e]);
-              dkr[c][e] = fmaf(ds, qf[c][e], dkr[c][e]);
-              dvr[c][e] = fmaf(pw, df[c][e], dvr[c][e]);
-            }
-        }
-        if (valid) {
-#pragma unroll
-          for (int c = 0; c < CH; ++c) {
-#pragma unroll
-            for (int e = 0; e < 8; ++e) dkr[c][e] *= p.scale;
-            uint4* gk4 = reinterpret_cast<uint4*>(dkb + (int64_t)key * p.dkd.st + (sub + 8 * c) * 8);
-            uint4* gv4 = reinterpret_cast<uint4*>(dvb + (int64_t)key * p.dvd.st + (sub + 8 * c) * 8);
-            if (p.acc_depth) {   // gradient cache shared by several layers: add to what earlier calls left
-              add8<T>(dkr[c], *gk4);
-              add8<T>(dvr[c], *gv4);
-            }
-            *gk4 = pack8<T>(dkr[c]);
-            *gv4 = pack8<T>(dvr[c]);
-          }
-        }
-      }
+    for (int j = 0; j < J; ++j) {
+      const uint4 k0 = tile_chunk<kRows>(kt, my_row, t4 + 4 * j), k1 = tile_chunk<kRows>(kt, 8 + my_row, t4 + 4 * j);
+      const uint32_t ka[4] = {k0.x, k1.x, k0.y, k1.y}, kb[4] = {k0.z, k1.z, k0.w, k1.w};
+      simt::Mma<T>::run(sc, ka, qa[j].x, qa[j].y);
+      simt::Mma<T>::run(sc, kb, qa[j].z, qa[j].w);
+      const uint4 v0 = tile_chunk<kRows>(vt, my_row, t4 + 4 * j), v1 = tile_chunk<kRows>(vt, 8 + my_row, t4 + 4 * j);
+      const uint32_t va[4] = {v0.x, v1.x, v0.y, v1.y}, vb[4] = {v0.z, v1.z, v0.w, v1.w};
+      simt::Mma<T>::run(dp, va, da[j].x, da[j].y);
+      simt::Mma<T>::run(dp, vb, da[j].z, da[j].w);
     }
+    // left operands P^T and scale dS^T: rows my_row, my_row + 8; contracted index = queries, then the
+    // queries again with what the rounding left over
+    uint32_t pt[4], dt[4];
 #pragma unroll
-    for (int g = 0; g < G; ++g) {
+    for (int nt = 0; nt < 2; ++nt) {
+      const bool live = my_row + 8 * nt < left;
+      float pw[2], ds[2];
 #pragma unroll
-      for (int c = 0; c < CH; ++c)
-#pragma unroll
-        for (int e = 0; e < 8; ++e) dq[g][c][e] = cross4_sum(dq[g][c][e]) * p.scale;
-      if (grp == 0) {
-        T* qp = reinterpret_cast<T*>(p.dq.ptr) + p.dq.off(b, t * G + g, h);
-#pragma unroll
-        for (int c = 0; c < CH; ++c) *reinterpret_cast<uint4*>(qp + (sub + 8 * c) * 8) = pack8<T>(dq[g][c]);
+      for (int c = 0; c < 2; ++c) {
+        pw[c] = live ? fast_exp2(fmaf(sc[2 * nt + c], p.scale_log2, -lse[c])) : 0.f;
+        ds[c] = live ? pw[c] * (dp[2 * nt + c] - delta[c]) * p.scale : 0.f;
       }
+      split_pair<T>(pw[0], pw[1], pt[nt], pt[nt + 2]);
+      split_pair<T>(ds[0], ds[1], dt[nt], dt[nt + 2]);
     }
+    {   // dQ^T += K^T (scale dS)^T
+      const uint32_t hi[2] = {transpose8x8(dt[0]), transpose8x8(dt[1])}, lo[2] = {transpose8x8(dt[2]), transpose8x8(dt[3])};
+#pragma unroll
+      for (int i = 0; i < I; ++i) add_transposed<T, kOne>(dq[i], kt, i, g, t4, left, hi, lo);
+    }
+    // The gradient rows take the place of the K and V rows and leave as a tile: stored from registers, a
+    // lane's 16 bytes beside three others', every instruction would write half lines.
+    __syncwarp();                                   // the K and V rows have been read by every lane
+    unsigned char* out = ring.tiles + (kt - ring.tiles);
+    T* dkb = reinterpret_cast<T*>(p.dkd.ptr) + p.dkd.off(s.b, (int64_t)s.t * p.Ls + s.l0 + my_row, s.h) + 8 * t4;
+    T* dvb = reinterpret_cast<T*>(p.dvd.ptr) + p.dvd.off(s.b, (int64_t)s.t * p.Ls + s.l0 + my_row, s.h) + 8 * t4;
+#pragma unroll
+    for (int j = 0; j < J; ++j) {
+      const uint32_t qw[4] = {qa[j].x, qa[j].y, qa[j].z, qa[j].w}, dw[4] = {da[j].x, da[j].y, da[j].z, da[j].w};
+      float gk[2][8], gv[2][8];                     // tile rows my_row, my_row + 8; chunk t + 4 j
+#pragma unroll
+      for (int w = 0; w < 4; ++w) {
+        float ck[4] = {0.f, 0.f, 0.f, 0.f}, cv[4] = {0.f, 0.f, 0.f, 0.f};
+        const uint32_t qb = transpose8x8(qw[w]), db = transpose8x8(dw[w]);
+        simt::Mma<T>::run(ck, dt, qb, qb);
+        simt::Mma<T>::run(cv, pt, db, db);
+#pragma unroll
+        for (int x = 0; x < 4; ++x) {
+          gk[x >> 1][2 * w + (x & 1)] = ck[x];
+          gv[x >> 1][2 * w + (x & 1)] = cv[x];
+        }
+      }
+#pragma unroll
+      for (int nt = 0; nt < 2; ++nt)
+        if (my_row + 8 * nt < left) {
+          if (kAdd) {   // gradient cache shared by several layers: add to what earlier calls left
+            add8<T>(gk[nt], *reinterpret_cast<const uint4*>(dkb + 8 * nt * p.dkd.st + 32 * j));
+            add8<T>(gv[nt], *reinterpret_cast<const uint4*>(dvb + 8 * nt * p.dvd.st + 32 * j));
+          }
+          *reinterpret_cast<uint4*>(out + chunk_at<kRows>(my_row + 8 * nt, t4 + 4 * j)) = pack8<T>(gk[nt]);
+          *reinterpret_cast<uint4*>(out + tile_bytes<D>() + chunk_at<kRows>(my_row + 8 * nt, t4 + 4 * j)) = pack8<T>(gv[nt]);
+        }
+    }
+    ring.store(p, omaps, s);
+
+    if (kOne || left <= kRows) {
+      T* qp = reinterpret_cast<T*>(p.dq.ptr) + p.dq.off(s.b, s.t * p.G + 2 * t4, s.h) + 8 * g;
+#pragma unroll
+      for (int c = 0; c < 2; ++c)
+        if (2 * t4 + c < p.G)
+#pragma unroll
+          for (int i = 0; i < I; ++i) {
+            float f[8];
+#pragma unroll
+            for (int e = 0; e < 8; ++e) f[e] = dq[i][e][c];
+            *reinterpret_cast<uint4*>(qp + c * p.dq.st + 64 * i) = pack8<T>(f);
+          }
+    }
+    s = next;
   }
+  if (!ok) ring.drain();
+  ring.stored_read();                               // before the shared memory goes
 }
 
-// G query rows of a position are held in registers: up to 2 at D = 128, up to 4 at D = 64.
-inline bool bwd_supported(int G, int D) { return G == 1 || G == 2 || (G == 4 && D == 64); }
+// ------------------------------------------------------------------------- host side
+inline bool make_maps(Maps* m, OutMaps* om, const Params& p, int dtype, int D, bool is_bwd) {
+  memset(m, 0, sizeof(*m));
+  memset(om, 0, sizeof(*om));
+  const int64_t rows = (int64_t)p.T_kv * p.Ls;
+  const int tail = p.L % kRows, g8 = p.G < 8 ? p.G : 8;
+  if (p.L >= kRows && !(tc::make_map_rows(&m->k, p.kd, dtype, p.B, rows, p.H, D, kRows) && tc::make_map_rows(&m->v, p.vd, dtype, p.B, rows, p.H, D, kRows)))
+    return false;
+  if (tail != 0 && !(tc::make_map_rows(&m->kt, p.kd, dtype, p.B, rows, p.H, D, tail) && tc::make_map_rows(&m->vt, p.vd, dtype, p.B, rows, p.H, D, tail)))
+    return false;
+  if (!tc::make_map_rows(&m->q, p.q, dtype, p.B, p.T_q, p.H, D, g8, false)) return false;
+  if (is_bwd && p.L >= kRows && !(tc::make_map_rows(&om->dk, p.dkd, dtype, p.B, rows, p.H, D, kRows) && tc::make_map_rows(&om->dv, p.dvd, dtype, p.B, rows, p.H, D, kRows)))
+    return false;
+  if (is_bwd && tail != 0 && !(tc::make_map_rows(&om->dkt, p.dkd, dtype, p.B, rows, p.H, D, tail) && tc::make_map_rows(&om->dvt, p.dvd, dtype, p.B, rows, p.H, D, tail)))
+    return false;
+  return !is_bwd || (tc::make_map_rows(&m->dout, p.dout, dtype, p.B, p.T_q, p.H, D, g8, false) &&
+                     tc::make_map_rows(&m->o, p.o, dtype, p.B, p.T_q, p.H, D, g8, false));
+}
+
+// The backward keeps all query rows of a position in one group.
+inline bool bwd_supported(int G) { return G <= 8; }
 
 }  // namespace fda
 }  // namespace moda

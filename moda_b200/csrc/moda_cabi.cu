@@ -5,18 +5,19 @@
 
 #include <cuda_runtime.h>
 
+#include <algorithm>
+#include <atomic>
+
 #include "common.cuh"
 #include "profiler.cuh"
 #include "simt_mma_kernels.cuh"
-#include "fda_kernels.cuh"
 #include "depth_cache_kernels.cuh"
-#ifndef MODA_NO_TCGEN05
 #include "tc_kernels.cuh"
+#include "fda_kernels.cuh"
 #include "tc_bwd_kernels.cuh"
 #include "tc_fwd3_kernel.cuh"
 #include "tc_bwd_launch.cuh"
 #include "mma_rate_probe.cuh"
-#endif
 
 namespace {
 
@@ -86,6 +87,8 @@ void fill_common(Params& p, const moda_problem* pr) {
   p.scale_log2 = pr->scale * 1.4426950216f;
   p.Ls = (pr->depth_rows_per_pos > pr->L) ? pr->depth_rows_per_pos : pr->L;
   p.acc_depth = pr->accumulate_depth_grads != 0;
+  static std::atomic<uint32_t> calls{0};
+  p.launch_id = (int)(calls.fetch_add(1, std::memory_order_relaxed) & 0x7fffffffu) + 1;
 }
 
 int cuda_fail(cudaError_t e) { g_last_cuda_error = (int)e; return MODA_ERR_CUDA; }
@@ -171,7 +174,7 @@ int simt_bwd_d(const Params& p, int D, int n_sm, cudaStream_t st) {
 // ----------------------------------------------------------------- depth-only (FDA) bandwidth path
 bool use_fda(const moda_problem* pr, bool is_bwd) {
   if (pr->mode != MODA_DEPTH_ONLY || pr->path != MODA_PATH_AUTO) return false;
-  return !is_bwd || fda::bwd_supported(pr->G, pr->D);
+  return !is_bwd || fda::bwd_supported(pr->G);
 }
 
 // Own-position depth (parallel_moda, causal or not) with one query row per position (G = 1) as
@@ -186,7 +189,7 @@ bool use_fda(const moda_problem* pr, bool is_bwd) {
 bool split_depth(const moda_problem* pr, bool is_bwd) {
   if (pr->path != MODA_PATH_AUTO || pr->L <= 0 || pr->G != 1) return false;
   if (pr->mode != MODA_CAUSAL && pr->mode != MODA_NONCAUSAL) return false;
-  return !is_bwd || fda::bwd_supported(pr->G, pr->D);
+  return !is_bwd || fda::bwd_supported(pr->G);
 }
 Params sequence_part(const Params& p) {
   Params s = p;
@@ -203,54 +206,53 @@ moda_problem attention_problem(const moda_problem* pr, bool is_bwd) {
   return a;
 }
 
-template <typename T, int D>
-int fda_fwd(const Params& p, int n_sm, cudaStream_t st) {
-  const int64_t units = (int64_t)p.B * p.T_kv * p.H;
-  const int64_t want = (units + 7) / 8, cap = (int64_t)n_sm * 32;
-  const int blocks = (int)(want < cap ? want : cap);
+// Warps of the bandwidth kernels walk the units with the stride of the grid.  A grid of just the blocks
+// that fit lets warps drift apart over a long launch and the sweep through memory with them; blocks
+// that end and are replaced keep it together (D = 128, L = 32, 1 M units, backward: 6.12 ms with one
+// round of blocks, 5.92 with 4, 5.42 with 64).  A block pays for its set-up with at least 8 steps a warp.
+template <typename K, typename... Args>
+int fda_launch(K kernel, int id, size_t smem, int n_sm, cudaStream_t st, const Params& p, const Args&... args) {
+  if (int rc = opt_in_smem(kernel, smem)) return rc;
+  int per_sm = 0;
+  MODA_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, fda::kWarps * 32, smem));
+  const int64_t units = (int64_t)p.B * p.T_kv * p.H, steps = units * ((p.L + fda::kRows - 1) / fda::kRows);
+  const int64_t fit = (int64_t)n_sm * per_sm, want = (units + fda::kWarps - 1) / fda::kWarps;
+  const int64_t rounds = std::min<int64_t>(64, std::max<int64_t>(1, steps / (fit * fda::kWarps * 8)));
   {
-    prof::Scope ps(prof::kFdaFwd, st);
-    fda::fwd_kernel<T, D><<<blocks, 256, 0, st>>>(p);
+    prof::Scope ps(id, st);
+    kernel<<<(int)std::min(want, fit * rounds), fda::kWarps * 32, smem, st>>>(p, args...);
   }
   MODA_CUDA(cudaGetLastError());
   g_last_launches += 1;
   return MODA_OK;
 }
-
-template <typename T, int D>
-int fda_bwd(const Params& p, int n_sm, cudaStream_t st) {
-  const int64_t units = (int64_t)p.B * p.T_kv * p.H;
-  const int64_t want = (units + 3) / 4, cap = (int64_t)n_sm * 64;
-  const int blocks = (int)(want < cap ? want : cap);
-  {
-    prof::Scope ps(prof::kFdaBwd, st);
-    if (p.G == 1) fda::bwd_kernel<T, D, 1><<<blocks, 128, 0, st>>>(p);
-    else if (p.G == 2) fda::bwd_kernel<T, D, 2><<<blocks, 128, 0, st>>>(p);
-    else if constexpr (D == 64) fda::bwd_kernel<T, D, 4><<<blocks, 128, 0, st>>>(p);
-  }
-  MODA_CUDA(cudaGetLastError());
-  g_last_launches += 1;
-  return MODA_OK;
+template <typename T, int D, bool kOne>
+int fda_run(const Params& p, const fda::Maps& maps, const fda::OutMaps& omaps, bool is_bwd, int n_sm, cudaStream_t st) {
+  if (!is_bwd) return fda_launch(fda::fwd_kernel<T, D, kOne>, prof::kFdaFwd, fda::smem_bytes<D, 1>(p.G), n_sm, st, p, maps);
+  return fda_launch(p.acc_depth ? fda::bwd_kernel<T, D, kOne, true> : fda::bwd_kernel<T, D, kOne, false>, prof::kFdaBwd,
+                    fda::smem_bytes<D, 3>(p.G), n_sm, st, p, maps, omaps);
 }
-
 template <typename T>
-int fda_dispatch(const Params& p, int D, bool is_bwd, int n_sm, cudaStream_t st) {
-  if (is_bwd) return D == 64 ? fda_bwd<T, 64>(p, n_sm, st) : fda_bwd<T, 128>(p, n_sm, st);
-  return D == 64 ? fda_fwd<T, 64>(p, n_sm, st) : fda_fwd<T, 128>(p, n_sm, st);
+int fda_run_d(const Params& p, const fda::Maps& m, const fda::OutMaps& om, int D, bool is_bwd, int n_sm, cudaStream_t st) {
+  const bool one = p.L <= fda::kRows;
+  if (D == 64) return one ? fda_run<T, 64, true>(p, m, om, is_bwd, n_sm, st) : fda_run<T, 64, false>(p, m, om, is_bwd, n_sm, st);
+  return one ? fda_run<T, 128, true>(p, m, om, is_bwd, n_sm, st) : fda_run<T, 128, false>(p, m, om, is_bwd, n_sm, st);
+}
+int fda_dispatch(const Params& p, const moda_problem* prob, bool is_bwd, int n_sm, cudaStream_t st) {
+  fda::Maps maps;
+  fda::OutMaps omaps;
+  if (!fda::make_maps(&maps, &omaps, p, prob->dtype, prob->D, is_bwd)) return MODA_ERR_UNSUPPORTED;
+  return prob->dtype == MODA_BF16 ? fda_run_d<__nv_bfloat16>(p, maps, omaps, prob->D, is_bwd, n_sm, st)
+                                  : fda_run_d<__half>(p, maps, omaps, prob->D, is_bwd, n_sm, st);
 }
 
 int resolve_path(const moda_problem* pr, bool is_bwd) {
-#ifndef MODA_NO_TCGEN05
   const bool ok = is_bwd ? tc::bwd_supported(pr) : tc::fwd_supported(pr);
-#else
-  const bool ok = false;
-#endif
   if (pr->path == MODA_PATH_SIMT_MMA) return MODA_PATH_SIMT_MMA;
   if (pr->path >= MODA_PATH_TCGEN05) return ok ? MODA_PATH_TCGEN05 : -MODA_ERR_UNSUPPORTED;
   return ok ? MODA_PATH_TCGEN05 : MODA_PATH_SIMT_MMA;
 }
 
-#ifndef MODA_NO_TCGEN05
 int tc_forward(const Params& p, const moda_problem* prob, int n_sm, cudaStream_t st) {
   // Two forwards.  tc::fwd3 (two 128-row query tiles per CTA, one CTA per SM, one MMA warp
   // ordering the work of both tiles) is the faster one once its grid fills the GPU; tc::fwd
@@ -265,7 +267,6 @@ int tc_forward(const Params& p, const moda_problem* prob, int n_sm, cudaStream_t
   if (two_tiles) return tc::fwd3(p, prob, st, &g_last_launches, &g_last_cuda_error);
   return tc::fwd(p, prob, st, &g_last_launches, &g_last_cuda_error);
 }
-#endif
 
 size_t delta_bytes(const moda_problem* pr) {
   const size_t n = (size_t)pr->B * pr->T_kv * pr->G * pr->H * sizeof(float);
@@ -358,16 +359,12 @@ int moda_b200_fwd(const moda_problem* prob, const moda_tensor4* q, const moda_te
   const int n_sm = sm_count(prob->device);
   if (n_sm <= 0) return cuda_fail(cudaErrorInvalidDevice);
   if (use_fda(prob, false))
-    return prob->dtype == MODA_BF16 ? fda_dispatch<__nv_bfloat16>(p, prob->D, false, n_sm, st)
-                                    : fda_dispatch<__half>(p, prob->D, false, n_sm, st);
+    return fda_dispatch(p, prob, false, n_sm, st);
   if (split_depth(prob, false)) {
-    if (int rc = prob->dtype == MODA_BF16 ? fda_dispatch<__nv_bfloat16>(p, prob->D, false, n_sm, st)
-                                          : fda_dispatch<__half>(p, prob->D, false, n_sm, st)) return rc;
+    if (int rc = fda_dispatch(p, prob, false, n_sm, st)) return rc;
     p = sequence_part(p);
   }
-#ifndef MODA_NO_TCGEN05
   if (path == MODA_PATH_TCGEN05) return tc_forward(p, &att, n_sm, st);
-#endif
   return prob->dtype == MODA_BF16 ? simt_fwd_d<__nv_bfloat16>(p, prob->D, st)
                                   : simt_fwd_d<__half>(p, prob->D, st);
 }
@@ -376,10 +373,8 @@ int moda_b200_bwd_workspace_bytes(const moda_problem* prob, size_t* bytes) {
   if (bytes == nullptr) return MODA_ERR_NULL;
   if (int rc = check_problem(prob)) return rc;
   size_t n = delta_bytes(prob);
-#ifndef MODA_NO_TCGEN05
   const moda_problem att = attention_problem(prob, true);
   n += tc::bwd_extra_workspace_bytes(&att);
-#endif
   *bytes = n;
   return MODA_OK;
 }
@@ -434,19 +429,15 @@ int moda_b200_bwd(const moda_problem* prob, const moda_tensor4* q, const moda_te
   const int n_sm = sm_count(prob->device);
   if (n_sm <= 0) return cuda_fail(cudaErrorInvalidDevice);
   if (use_fda(prob, true))
-    return prob->dtype == MODA_BF16 ? fda_dispatch<__nv_bfloat16>(p, prob->D, true, n_sm, st)
-                                    : fda_dispatch<__half>(p, prob->D, true, n_sm, st);
+    return fda_dispatch(p, prob, true, n_sm, st);
   if (split_depth(prob, true)) {   // depth rows' dq share, d_depth_k, d_depth_v; then the sequence part
-    if (int rc = prob->dtype == MODA_BF16 ? fda_dispatch<__nv_bfloat16>(p, prob->D, true, n_sm, st)
-                                          : fda_dispatch<__half>(p, prob->D, true, n_sm, st)) return rc;
+    if (int rc = fda_dispatch(p, prob, true, n_sm, st)) return rc;
     p = sequence_part(p);
   }
-#ifndef MODA_NO_TCGEN05
   if (path == MODA_PATH_TCGEN05) {
     void* extra = reinterpret_cast<unsigned char*>(workspace) + delta_bytes(prob);
     return tc::bwd(p, &att, extra, n_sm, st, &g_last_launches, &g_last_cuda_error);
   }
-#endif
   return prob->dtype == MODA_BF16 ? simt_bwd_d<__nv_bfloat16>(p, prob->D, n_sm, st)
                                   : simt_bwd_d<__half>(p, prob->D, n_sm, st);
 }
@@ -499,14 +490,10 @@ const char* moda_b200_kernel_name(int kernel_id) { return prof::kernel_name(kern
 
 int moda_b200_device_status(int* status) {
   if (status == nullptr) return MODA_ERR_NULL;
-#ifndef MODA_NO_TCGEN05
   int v = 0;
   const int e = tc::read_status(&v);
   if (e != 0) { g_last_cuda_error = e; return MODA_ERR_CUDA; }
   *status = v;
-#else
-  *status = 0;
-#endif
   return MODA_OK;
 }
 
@@ -558,7 +545,6 @@ int moda_b200_tensor_pipe_rates(int device, float* clocks_per_mma, void* stream)
   DeviceGuard guard(device);
   if (!guard.ok) return cuda_fail(guard.err);
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-  MODA_CUDA(tc::clear_launch_status(st));
   MODA_CUDA(tc::mma_rates(clocks_per_mma, st));
   g_last_launches = 12;
   return MODA_OK;

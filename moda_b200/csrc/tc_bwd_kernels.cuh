@@ -180,7 +180,7 @@ dq_kernel(const __grid_constant__ Params p, const __grid_constant__ DqMaps maps,
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   const uint32_t base = smem_u32(smem_raw);
   if (base & 1023u) {   // the 128-byte swizzle needs 1024-byte aligned tiles
-    if (threadIdx.x == 0) record_failure(2 << 8);
+    if (threadIdx.x == 0) record_failure(2 << 8, p.launch_id);
     return;
   }
   const uint32_t sRing = base;
@@ -191,10 +191,10 @@ dq_kernel(const __grid_constant__ Params p, const __grid_constant__ DqMaps maps,
   unsigned char* gctl = smem_raw + ctl_off;
   volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(gctl + 8 * kMaxBars);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(gctl + 8 * kMaxBars + 4);
-  volatile int* drain_flag = reinterpret_cast<volatile int*>(gctl + 8 * kMaxBars + 8);
+  volatile int* drain_flag = reinterpret_cast<volatile int*>(gctl + 8 * kMaxBars + 12);
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  if (*reinterpret_cast<volatile int*>(&g_tc_status) != 0) return;
+  if (launch_failed(p)) return;
 
   const int n_qt = (p.T_q + kBM - 1) / kBM;
   const BlockId bid = block_order(p, D);
@@ -231,8 +231,8 @@ dq_kernel(const __grid_constant__ Params p, const __grid_constant__ DqMaps maps,
       mbar_init(bars + 8 * (B_.p0 + i), 128);
       mbar_init(bars + 8 * (B_.r0 + i), 128); mbar_init(bars + 8 * (B_.t0 + i), 1);
     }
-    *abort_flag = 0;
-    *drain_flag = 0;
+    arm_abort(abort_flag, p);
+    arm_abort(drain_flag, p);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   }
@@ -521,7 +521,7 @@ dkv_kernel(const __grid_constant__ Params p, const __grid_constant__ DkvMaps map
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   const uint32_t base = smem_u32(smem_raw);
   if (base & 1023u) {
-    if (threadIdx.x == 0) record_failure(2 << 8);
+    if (threadIdx.x == 0) record_failure(2 << 8, p.launch_id);
     return;
   }
   const uint32_t sRing = base;
@@ -534,10 +534,10 @@ dkv_kernel(const __grid_constant__ Params p, const __grid_constant__ DkvMaps map
   unsigned char* gctl = smem_raw + ctl_off;
   volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(gctl + 8 * kMaxBars);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(gctl + 8 * kMaxBars + 4);
-  volatile int* drain_flag = reinterpret_cast<volatile int*>(gctl + 8 * kMaxBars + 8);
+  volatile int* drain_flag = reinterpret_cast<volatile int*>(gctl + 8 * kMaxBars + 12);
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  if (*reinterpret_cast<volatile int*>(&g_tc_status) != 0) return;
+  if (launch_failed(p)) return;
 
   const BlockId bid = block_order(p, D);
   const int h = bid.h, b = bid.b;
@@ -570,8 +570,8 @@ dkv_kernel(const __grid_constant__ Params p, const __grid_constant__ DkvMaps map
       mbar_init(bars + 8 * (B_.p0 + i), 128);
       mbar_init(bars + 8 * (B_.r0 + i), 128); mbar_init(bars + 8 * (B_.t0 + i), 1);
     }
-    *abort_flag = 0;
-    *drain_flag = 0;
+    arm_abort(abort_flag, p);
+    arm_abort(drain_flag, p);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   }
@@ -898,7 +898,7 @@ depth_grad_kernel(const __grid_constant__ Params p, const __grid_constant__ DkvM
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   const uint32_t base = smem_u32(smem_raw);
   if (base & 1023u) {
-    if (threadIdx.x == 0) record_failure(2 << 8);
+    if (threadIdx.x == 0) record_failure(2 << 8, p.launch_id);
     return;
   }
   const uint32_t sQ = base, sDO = base + kStepTile, sStat = base + 2 * kStepTile;
@@ -909,10 +909,10 @@ depth_grad_kernel(const __grid_constant__ Params p, const __grid_constant__ DkvM
   unsigned char* gctl = smem_raw + ctl_off;
   volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(gctl + 104);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(gctl + 108);
-  volatile int* drain_flag = reinterpret_cast<volatile int*>(gctl + 112);
+  volatile int* drain_flag = reinterpret_cast<volatile int*>(gctl + 116);
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  if (*reinterpret_cast<volatile int*>(&g_tc_status) != 0) return;
+  if (launch_failed(p)) return;
 
   const int n_xb = (p.T_q + kStep - 1) / kStep;
   const int total = n_xb * p.H * p.B;                   // 64-row blocks; this CTA takes blockIdx.x, + gridDim.x, ...
@@ -929,8 +929,8 @@ depth_grad_kernel(const __grid_constant__ Params p, const __grid_constant__ DkvM
     mbar_init(bars + 8 * kDgU, 1);
     mbar_init(bars + 8 * kDgE, 256);
     mbar_init(bars + 8 * kDgQFree, 1);
-    *abort_flag = 0;
-    *drain_flag = 0;
+    arm_abort(abort_flag, p);
+    arm_abort(drain_flag, p);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   }

@@ -192,14 +192,12 @@ inline int bwd(const Params& p, const moda_problem* pr, void* extra, int n_sm, c
     return MODA_ERR_UNSUPPORTED;
   if ((int64_t)((p.T_q + kStep - 1) / kStep) * p.H * p.B > 0x7fffffff || n_sm <= 0) return MODA_ERR_UNSUPPORTED;
 
-  cudaError_t e = clear_launch_status(st);
-  if (e == cudaSuccess) {
-    const bool bf = dt == MODA_BF16;
-    if (D == 128) e = bf ? launch_bwd<__nv_bfloat16, 128>(p, m, w, T_qp, dg, fused, n_sm, st, launches)
-                         : launch_bwd<__half, 128>(p, m, w, T_qp, dg, fused, n_sm, st, launches);
-    else e = bf ? launch_bwd<__nv_bfloat16, 64>(p, m, w, T_qp, dg, false, n_sm, st, launches)
-                : launch_bwd<__half, 64>(p, m, w, T_qp, dg, false, n_sm, st, launches);
-  }
+  cudaError_t e;
+  const bool bf = dt == MODA_BF16;
+  if (D == 128) e = bf ? launch_bwd<__nv_bfloat16, 128>(p, m, w, T_qp, dg, fused, n_sm, st, launches)
+                       : launch_bwd<__half, 128>(p, m, w, T_qp, dg, fused, n_sm, st, launches);
+  else e = bf ? launch_bwd<__nv_bfloat16, 64>(p, m, w, T_qp, dg, false, n_sm, st, launches)
+              : launch_bwd<__half, 64>(p, m, w, T_qp, dg, false, n_sm, st, launches);
   if (e != cudaSuccess) { *cuda_err = (int)e; return MODA_ERR_CUDA; }
   return MODA_OK;
 }

@@ -125,7 +125,7 @@ fwd3_kernel(const __grid_constant__ Params p, const __grid_constant__ Fwd3Maps m
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   const uint32_t base = smem_u32(smem_raw);
   if (base & 1023u) {
-    if (threadIdx.x == 0) record_failure(2 << 8);
+    if (threadIdx.x == 0) record_failure(2 << 8, p.launch_id);
     return;
   }
   const uint32_t sQ = base;                              // Q_a at sQ + a * kTile
@@ -137,10 +137,10 @@ fwd3_kernel(const __grid_constant__ Params p, const __grid_constant__ Fwd3Maps m
   unsigned char* gctl = smem_raw + ctl_off;
   volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(gctl + 8 * kMaxBars);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(gctl + 8 * kMaxBars + 4);
-  volatile int* drain_flag = reinterpret_cast<volatile int*>(gctl + 8 * kMaxBars + 8);
+  volatile int* drain_flag = reinterpret_cast<volatile int*>(gctl + 8 * kMaxBars + 12);
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  if (*reinterpret_cast<volatile int*>(&g_tc_status) != 0) return;
+  if (launch_failed(p)) return;
 
   const int n_pairs = (p.T_q + 2 * kBM - 1) / (2 * kBM);
   const BlockId bid = block_order(p, D);
@@ -164,8 +164,8 @@ fwd3_kernel(const __grid_constant__ Params p, const __grid_constant__ Fwd3Maps m
       mbar_init(bars + 8 * (B_::s0 + i), 1);
       for (int j = 0; j < kF3Parts; ++j) mbar_init(bars + 8 * (B_::p0 + 2 * j + i), 4);   // one arrival per softmax warp
     }
-    *abort_flag = 0;
-    *drain_flag = 0;
+    arm_abort(abort_flag, p);
+    arm_abort(drain_flag, p);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   }
@@ -500,8 +500,7 @@ inline int fwd3(const Params& p, const moda_problem* pr, cudaStream_t st, int* l
   FwdMaps fm;
   if (!make_fwd_maps(&fm, p, pr)) return MODA_ERR_UNSUPPORTED;
   Fwd3Maps maps{fm.q, fm.k, fm.v, fm.kd, fm.vd};
-  cudaError_t e = clear_launch_status(st);
-  if (e != cudaSuccess) { *cuda_err = (int)e; return MODA_ERR_CUDA; }
+  cudaError_t e;
   const bool bf = pr->dtype == MODA_BF16;
   if (pr->D == 128) e = bf ? launch_fwd3<__nv_bfloat16, 128>(p, maps, st) : launch_fwd3<__half, 128>(p, maps, st);
   else e = bf ? launch_fwd3<__nv_bfloat16, 64>(p, maps, st) : launch_fwd3<__half, 64>(p, maps, st);

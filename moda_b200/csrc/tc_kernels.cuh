@@ -49,16 +49,26 @@ constexpr uint32_t kHalfBytes = 128 * 64 * 2;  // one TMA box: [128 rows x 64 el
 constexpr uint32_t kTileBytes = 2 * kHalfBytes; // a [128 x 128] 16-bit tile (two boxes)
 template <int D> __host__ __device__ constexpr uint32_t tile_bytes() { return (uint32_t)(D / 64) * kHalfBytes; }   // [128 x D]
 
-// 0 = ok; otherwise (code << 8) | barrier id of the first wait that expired.  g_tc_status is the
-// abort flag of the launch in flight: it is cleared when a launch is enqueued and lets the CTAs
-// that start after a failure return at once.  g_tc_sticky keeps the first failure of any launch
-// until the host reads it (moda_b200_device_status), so that a later call cannot erase it.
-__device__ int g_tc_status;
+// g_tc_failed is the number (Params::launch_id) of the call in which a wait expired last: the CTAs of
+// that call's launches which start after the failure return at once, and later calls, whose numbers
+// differ, need nothing cleared before they are enqueued.  g_tc_sticky keeps the first failure of any
+// launch, (code << 8) | barrier id of the wait that expired, until the host reads it
+// (moda_b200_device_status), so that a later call cannot erase it.
+__device__ int g_tc_failed;
 __device__ int g_tc_sticky;
 
-__device__ __forceinline__ void record_failure(int code) {
-  atomicCAS(&g_tc_status, 0, code);
+__device__ __forceinline__ void record_failure(int code, int launch_id) {
+  atomicExch(&g_tc_failed, launch_id);
   atomicCAS(&g_tc_sticky, 0, code);
+}
+
+__device__ __forceinline__ bool launch_failed(const Params& p) {
+  return *reinterpret_cast<volatile int*>(&g_tc_failed) == p.launch_id;
+}
+// An abort word in shared memory and, behind it, the call's number for whoever sets it.
+__device__ __forceinline__ void arm_abort(volatile int* flag, const Params& p) {
+  flag[0] = 0;
+  flag[1] = p.launch_id;
 }
 
 struct FwdMaps { CUtensorMap q, k, v, kd, vd; };
@@ -103,7 +113,7 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
     if (*abort_flag != 0) return false;
   }
   *abort_flag = 1;
-  record_failure((1 << 8) | bar_id);
+  record_failure((1 << 8) | bar_id, abort_flag[1]);
   return false;
 }
 
@@ -391,10 +401,10 @@ fwd_kernel(const __grid_constant__ Params p, const __grid_constant__ FwdMaps map
   const uint32_t bars = ctl;                                    // kBarCount x 8 bytes
   volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(gctl + 64);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(gctl + 72);
-  volatile int* drain_flag = reinterpret_cast<volatile int*>(gctl + 76);   // never set: lets the drain waits run
+  volatile int* drain_flag = reinterpret_cast<volatile int*>(gctl + 80);   // never set: lets the drain waits run
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  if (*reinterpret_cast<volatile int*>(&g_tc_status) != 0) return;   // an earlier CTA failed: do nothing
+  if (launch_failed(p)) return;   // an earlier CTA failed: do nothing
 
   const int n_qt = (p.T_q + kBM - 1) / kBM;
   const BlockId bid = block_order(p, D);
@@ -414,8 +424,8 @@ fwd_kernel(const __grid_constant__ Params p, const __grid_constant__ FwdMaps map
     mbar_init(bars + 8 * kBarO, 1);
     mbar_init(bars + 8 * kBarKFree, 1);
     mbar_init(bars + 8 * kBarVFree, 1);
-    *abort_flag = 0;
-    *drain_flag = 0;
+    arm_abort(abort_flag, p);
+    arm_abort(drain_flag, p);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   }
@@ -625,8 +635,8 @@ inline EncodeTiledFn encode_fn() {
 // [B, T, H, D] view -> 4-D tensor map (D, H, T, B), box [64, 1, box_rows, 1], 128B swizzle, zero
 // fill.  A dimension of extent 1 may carry any stride (it is never multiplied by a non-zero
 // index) and gets a placeholder TMA accepts; every other stride must be a positive multiple of
-// 8 elements, which the entry points have checked.
-inline bool make_map_rows(CUtensorMap* m, const View& v, int dtype, int B, int64_t T, int H, int D, int box_rows) {
+// 8 elements, which the entry points have checked.  !swizzled: box [D, 1, box_rows, 1], rows stored as they are.
+inline bool make_map_rows(CUtensorMap* m, const View& v, int dtype, int B, int64_t T, int H, int D, int box_rows, bool swizzled = true) {
   EncodeTiledFn fn = encode_fn();
   if (fn == nullptr || v.ptr == nullptr) return false;
   bool bad = false;
@@ -638,10 +648,10 @@ inline bool make_map_rows(CUtensorMap* m, const View& v, int dtype, int B, int64
   cuuint64_t dims[4] = {(cuuint64_t)D, (cuuint64_t)H, (cuuint64_t)T, (cuuint64_t)B};
   cuuint64_t strides[3] = {stride(v.sh, H), stride(v.st, T), stride(v.sb, B)};
   if (bad) return false;
-  cuuint32_t box[4] = {64, 1, (cuuint32_t)box_rows, 1};
+  cuuint32_t box[4] = {(cuuint32_t)(swizzled ? 64 : D), 1, (cuuint32_t)box_rows, 1};
   cuuint32_t estr[4] = {1, 1, 1, 1};
   return fn(m, dtype == MODA_BF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 4, v.ptr,
-            dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+            dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, swizzled ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE,
             CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
@@ -676,14 +686,6 @@ inline bool fwd_supported(const moda_problem* pr) {
   return (pr->D == 128 || pr->D == 64) && pr->mode != MODA_DEPTH_ONLY && pr->scale > 0.f && depth_layout_supported(pr);
 }
 
-// Clears the abort flag of the launch about to be enqueued (the sticky word is left alone).
-inline cudaError_t clear_launch_status(cudaStream_t st) {
-  void* status_addr = nullptr;
-  cudaError_t e = cudaGetSymbolAddress(&status_addr, g_tc_status);
-  if (e == cudaSuccess) e = cudaMemsetAsync(status_addr, 0, sizeof(int), st);
-  return e;
-}
-
 inline bool make_fwd_maps(FwdMaps* maps, const Params& p, const moda_problem* pr) {
   memset(maps, 0, sizeof(*maps));
   const int D = pr->D;
@@ -713,8 +715,7 @@ inline cudaError_t launch_fwd(const Params& p, const FwdMaps& maps, cudaStream_t
 inline int fwd(const Params& p, const moda_problem* pr, cudaStream_t st, int* launches, int* cuda_err) {
   FwdMaps maps;
   if (!make_fwd_maps(&maps, p, pr)) return MODA_ERR_UNSUPPORTED;
-  cudaError_t e = clear_launch_status(st);
-  if (e != cudaSuccess) { *cuda_err = (int)e; return MODA_ERR_CUDA; }
+  cudaError_t e;
   const bool bf = pr->dtype == MODA_BF16;
   if (pr->D == 128) e = bf ? launch_fwd<__nv_bfloat16, 128>(p, maps, st) : launch_fwd<__half, 128>(p, maps, st);
   else e = bf ? launch_fwd<__nv_bfloat16, 64>(p, maps, st) : launch_fwd<__half, 64>(p, maps, st);
@@ -731,6 +732,7 @@ inline int read_status(int* out) {
   if (v != 0) {
     const int zero = 0;
     e = cudaMemcpyToSymbol(g_tc_sticky, &zero, sizeof(int));
+    if (e == cudaSuccess) e = cudaMemcpyToSymbol(g_tc_failed, &zero, sizeof(int));   // a captured call may be replayed
     if (e != cudaSuccess) return (int)e;
   }
   *out = v;
