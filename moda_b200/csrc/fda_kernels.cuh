@@ -151,8 +151,8 @@ struct Ring {
     queries = smem + kWarps * 4 * tile_bytes<D>() + w * q_bytes;
     unsigned char* ctl = smem + kWarps * (4 * tile_bytes<D>() + q_bytes);
     bars = smem_u32(ctl) + w * 16;
-    abort_flag = reinterpret_cast<volatile int*>(ctl + kWarps * 16);     // {abort, call}, {drain, call}
-    if (threadIdx.x == 0) { tc::arm_abort(abort_flag, p); tc::arm_abort(abort_flag + 2, p); }
+    abort_flag = reinterpret_cast<volatile int*>(ctl + kWarps * 16);     // abort, drain
+    if (threadIdx.x == 0) abort_flag[0] = abort_flag[1] = 0;
     if ((threadIdx.x & 31) == 0) {
       tc::mbar_init(bars, 1);
       tc::mbar_init(bars + 8, 1);
@@ -212,7 +212,7 @@ struct Ring {
   }
   // After a failed wait: loads in flight land before the shared memory is given up.
   __device__ __forceinline__ void drain() {
-    for (int i = taken - 1; i < issued; ++i) tc::mbar_wait(bars + 8 * (i & 1), (i >> 1) & 1, abort_flag + 2, 30);
+    for (int i = taken - 1; i < issued; ++i) tc::mbar_wait(bars + 8 * (i & 1), (i >> 1) & 1, abort_flag + 1, 30);
   }
   __device__ __forceinline__ const unsigned char* stage() const { return tiles + ((taken - 1) & 1) * 2 * tile_bytes<D>(); }
 };
@@ -259,7 +259,7 @@ __global__ void __launch_bounds__(kWarps * 32, D == 64 ? 6 : 3) fwd_kernel(const
   constexpr int J = D / 32, I = D / 64;
   extern __shared__ __align__(1024) unsigned char smem[];
   if (smem_u32(smem) & 1023u) {                     // the swizzle is a function of the shared-memory address
-    if (threadIdx.x == 0) tc::record_failure(2 << 8, p.launch_id);
+    if (threadIdx.x == 0) tc::record_failure(2 << 8);
     return;
   }
   if (tc::launch_failed(p)) return;
@@ -368,7 +368,10 @@ __global__ void __launch_bounds__(kWarps * 32, D == 64 ? 6 : 3) fwd_kernel(const
     }
     s = next;
   }
-  if (!ok) ring.drain();
+  if (!ok) {
+    ring.drain();
+    tc::publish_failure(p, ring.abort_flag);
+  }
 }
 
 // ------------------------------------------------------------------------- backward
@@ -380,7 +383,7 @@ __global__ void __launch_bounds__(kWarps * 32, D == 64 ? (kOne ? 5 : 4) : 3) bwd
   constexpr int J = D / 32, I = D / 64;
   extern __shared__ __align__(1024) unsigned char smem[];
   if (smem_u32(smem) & 1023u) {
-    if (threadIdx.x == 0) tc::record_failure(2 << 8, p.launch_id);
+    if (threadIdx.x == 0) tc::record_failure(2 << 8);
     return;
   }
   if (tc::launch_failed(p)) return;
@@ -522,7 +525,10 @@ __global__ void __launch_bounds__(kWarps * 32, D == 64 ? (kOne ? 5 : 4) : 3) bwd
     }
     s = next;
   }
-  if (!ok) ring.drain();
+  if (!ok) {
+    ring.drain();
+    tc::publish_failure(p, ring.abort_flag);
+  }
   ring.stored_read();                               // before the shared memory goes
 }
 

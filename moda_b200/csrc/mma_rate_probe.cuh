@@ -24,7 +24,7 @@ __global__ void __launch_bounds__(128, 1) mma_rate_kernel(float* out) {
   extern __shared__ __align__(1024) unsigned char probe_smem[];
   __shared__ __align__(8) unsigned long long bar;
   __shared__ uint32_t tmem_slot;
-  __shared__ int abort_flag[2];     // {flag, call number}: no call has number -1
+  __shared__ int abort_flag;
   const uint32_t base = (smem_u32(probe_smem) + 1023u) & ~1023u;
   unsigned char* gbase = probe_smem + (base - smem_u32(probe_smem));
   const uint32_t sA = base, sB = base + 16384, bar_addr = smem_u32(&bar);
@@ -32,8 +32,7 @@ __global__ void __launch_bounds__(128, 1) mma_rate_kernel(float* out) {
   for (int i = threadIdx.x; i < (16384 + 32768) / 4; i += blockDim.x) reinterpret_cast<uint32_t*>(gbase)[i] = 0u;
   if (threadIdx.x == 0) {
     mbar_init(bar_addr, 1);
-    abort_flag[0] = 0;
-    abort_flag[1] = -1;
+    abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   }
@@ -72,7 +71,7 @@ __global__ void __launch_bounds__(128, 1) mma_rate_kernel(float* out) {
       tc_commit(bar_addr);
     }
     __syncwarp();
-    const bool ok = mbar_wait(bar_addr, 0, abort_flag, 0);
+    const bool ok = mbar_wait(bar_addr, 0, &abort_flag, 0);
     const unsigned t1 = clock();
     if (lane == 0) *out = ok ? (float)(t1 - t0) / kProbeMmas : -1.f;
   }

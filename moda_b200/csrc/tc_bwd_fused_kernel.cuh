@@ -147,7 +147,7 @@ bwd_fused_kernel(const __grid_constant__ Params p, const __grid_constant__ DkvMa
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   const uint32_t base = smem_u32(smem_raw);
   if (base & 1023u) {
-    if (threadIdx.x == 0) record_failure(2 << 8, p.launch_id);
+    if (threadIdx.x == 0) record_failure(2 << 8);
     return;
   }
   const uint32_t sK = base;                                   // [128 keys x 128] K tile, resident
@@ -162,7 +162,7 @@ bwd_fused_kernel(const __grid_constant__ Params p, const __grid_constant__ DkvMa
   unsigned char* gctl = smem_raw + ctl_off;
   volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(gctl + 8 * kMaxBars);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(gctl + 8 * kMaxBars + 4);
-  volatile int* drain_flag = reinterpret_cast<volatile int*>(gctl + 8 * kMaxBars + 12);
+  volatile int* drain_flag = reinterpret_cast<volatile int*>(gctl + 8 * kMaxBars + 8);
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   if (launch_failed(p)) return;
@@ -189,8 +189,8 @@ bwd_fused_kernel(const __grid_constant__ Params p, const __grid_constant__ DkvMa
       mbar_init(bars + 8 * (B_::ws0 + i), 128);
       mbar_init(bars + 8 * (B_::qd0 + i), 1);
     }
-    arm_abort(abort_flag, p);
-    arm_abort(drain_flag, p);
+    *abort_flag = 0;
+    *drain_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   }
@@ -476,6 +476,7 @@ bwd_fused_kernel(const __grid_constant__ Params p, const __grid_constant__ DkvMa
   }
   tc_fence_before();
   __syncthreads();
+  if (tid == 0) publish_failure(p, abort_flag);
   if (warp == 0) {
     tc_fence_after();
     tmem_dealloc(tmem, 512);

@@ -180,7 +180,7 @@ dq_kernel(const __grid_constant__ Params p, const __grid_constant__ DqMaps maps,
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   const uint32_t base = smem_u32(smem_raw);
   if (base & 1023u) {   // the 128-byte swizzle needs 1024-byte aligned tiles
-    if (threadIdx.x == 0) record_failure(2 << 8, p.launch_id);
+    if (threadIdx.x == 0) record_failure(2 << 8);
     return;
   }
   const uint32_t sRing = base;
@@ -191,7 +191,7 @@ dq_kernel(const __grid_constant__ Params p, const __grid_constant__ DqMaps maps,
   unsigned char* gctl = smem_raw + ctl_off;
   volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(gctl + 8 * kMaxBars);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(gctl + 8 * kMaxBars + 4);
-  volatile int* drain_flag = reinterpret_cast<volatile int*>(gctl + 8 * kMaxBars + 12);
+  volatile int* drain_flag = reinterpret_cast<volatile int*>(gctl + 8 * kMaxBars + 8);
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   if (launch_failed(p)) return;
@@ -231,8 +231,8 @@ dq_kernel(const __grid_constant__ Params p, const __grid_constant__ DqMaps maps,
       mbar_init(bars + 8 * (B_.p0 + i), 128);
       mbar_init(bars + 8 * (B_.r0 + i), 128); mbar_init(bars + 8 * (B_.t0 + i), 1);
     }
-    arm_abort(abort_flag, p);
-    arm_abort(drain_flag, p);
+    *abort_flag = 0;
+    *drain_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   }
@@ -490,6 +490,7 @@ dq_kernel(const __grid_constant__ Params p, const __grid_constant__ DqMaps maps,
   }
   tc_fence_before();
   __syncthreads();
+  if (tid == 0) publish_failure(p, abort_flag);
   if (warp == 0) {
     tc_fence_after();
     tmem_dealloc(tmem, 512);
@@ -521,7 +522,7 @@ dkv_kernel(const __grid_constant__ Params p, const __grid_constant__ DkvMaps map
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   const uint32_t base = smem_u32(smem_raw);
   if (base & 1023u) {
-    if (threadIdx.x == 0) record_failure(2 << 8, p.launch_id);
+    if (threadIdx.x == 0) record_failure(2 << 8);
     return;
   }
   const uint32_t sRing = base;
@@ -534,7 +535,7 @@ dkv_kernel(const __grid_constant__ Params p, const __grid_constant__ DkvMaps map
   unsigned char* gctl = smem_raw + ctl_off;
   volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(gctl + 8 * kMaxBars);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(gctl + 8 * kMaxBars + 4);
-  volatile int* drain_flag = reinterpret_cast<volatile int*>(gctl + 8 * kMaxBars + 12);
+  volatile int* drain_flag = reinterpret_cast<volatile int*>(gctl + 8 * kMaxBars + 8);
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   if (launch_failed(p)) return;
@@ -570,8 +571,8 @@ dkv_kernel(const __grid_constant__ Params p, const __grid_constant__ DkvMaps map
       mbar_init(bars + 8 * (B_.p0 + i), 128);
       mbar_init(bars + 8 * (B_.r0 + i), 128); mbar_init(bars + 8 * (B_.t0 + i), 1);
     }
-    arm_abort(abort_flag, p);
-    arm_abort(drain_flag, p);
+    *abort_flag = 0;
+    *drain_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   }
@@ -828,6 +829,7 @@ dkv_kernel(const __grid_constant__ Params p, const __grid_constant__ DkvMaps map
   }
   tc_fence_before();
   __syncthreads();
+  if (tid == 0) publish_failure(p, abort_flag);
   if (warp == 0) {
     tc_fence_after();
     tmem_dealloc(tmem, 512);
@@ -898,7 +900,7 @@ depth_grad_kernel(const __grid_constant__ Params p, const __grid_constant__ DkvM
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   const uint32_t base = smem_u32(smem_raw);
   if (base & 1023u) {
-    if (threadIdx.x == 0) record_failure(2 << 8, p.launch_id);
+    if (threadIdx.x == 0) record_failure(2 << 8);
     return;
   }
   const uint32_t sQ = base, sDO = base + kStepTile, sStat = base + 2 * kStepTile;
@@ -909,7 +911,7 @@ depth_grad_kernel(const __grid_constant__ Params p, const __grid_constant__ DkvM
   unsigned char* gctl = smem_raw + ctl_off;
   volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(gctl + 104);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(gctl + 108);
-  volatile int* drain_flag = reinterpret_cast<volatile int*>(gctl + 116);
+  volatile int* drain_flag = reinterpret_cast<volatile int*>(gctl + 112);
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   if (launch_failed(p)) return;
@@ -929,8 +931,8 @@ depth_grad_kernel(const __grid_constant__ Params p, const __grid_constant__ DkvM
     mbar_init(bars + 8 * kDgU, 1);
     mbar_init(bars + 8 * kDgE, 256);
     mbar_init(bars + 8 * kDgQFree, 1);
-    arm_abort(abort_flag, p);
-    arm_abort(drain_flag, p);
+    *abort_flag = 0;
+    *drain_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   }
@@ -1187,6 +1189,7 @@ depth_grad_kernel(const __grid_constant__ Params p, const __grid_constant__ DkvM
   }
   tc_fence_before();
   __syncthreads();
+  if (tid == 0) publish_failure(p, abort_flag);
   if (warp == 0) {
     tc_fence_after();
     tmem_dealloc(tmem, 512);

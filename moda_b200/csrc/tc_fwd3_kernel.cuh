@@ -125,7 +125,7 @@ fwd3_kernel(const __grid_constant__ Params p, const __grid_constant__ Fwd3Maps m
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   const uint32_t base = smem_u32(smem_raw);
   if (base & 1023u) {
-    if (threadIdx.x == 0) record_failure(2 << 8, p.launch_id);
+    if (threadIdx.x == 0) record_failure(2 << 8);
     return;
   }
   const uint32_t sQ = base;                              // Q_a at sQ + a * kTile
@@ -137,7 +137,7 @@ fwd3_kernel(const __grid_constant__ Params p, const __grid_constant__ Fwd3Maps m
   unsigned char* gctl = smem_raw + ctl_off;
   volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(gctl + 8 * kMaxBars);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(gctl + 8 * kMaxBars + 4);
-  volatile int* drain_flag = reinterpret_cast<volatile int*>(gctl + 8 * kMaxBars + 12);
+  volatile int* drain_flag = reinterpret_cast<volatile int*>(gctl + 8 * kMaxBars + 8);
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   if (launch_failed(p)) return;
@@ -164,8 +164,8 @@ fwd3_kernel(const __grid_constant__ Params p, const __grid_constant__ Fwd3Maps m
       mbar_init(bars + 8 * (B_::s0 + i), 1);
       for (int j = 0; j < kF3Parts; ++j) mbar_init(bars + 8 * (B_::p0 + 2 * j + i), 4);   // one arrival per softmax warp
     }
-    arm_abort(abort_flag, p);
-    arm_abort(drain_flag, p);
+    *abort_flag = 0;
+    *drain_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   }
@@ -476,6 +476,7 @@ fwd3_kernel(const __grid_constant__ Params p, const __grid_constant__ Fwd3Maps m
   }
   tc_fence_before();
   __syncthreads();
+  if (tid == 0) publish_failure(p, abort_flag);
   if (warp == 0) {
     tc_fence_after();
     tmem_dealloc(tmem, 512);
