@@ -273,11 +273,14 @@ size_t delta_bytes(const moda_problem* pr) {
   return (n + 255) & ~(size_t)255;
 }
 
+// cudaSetDevice also where the device is the current one already: it makes the device's context current on
+// the calling thread, which an autograd thread that has neither allocated nor launched anything yet
+// lacks, and without one the driver refuses to encode a tensor map.
 struct DeviceGuard {
   int prev = -1; bool ok = true; cudaError_t err = cudaSuccess;
   explicit DeviceGuard(int dev) {
     err = cudaGetDevice(&prev);
-    if (err == cudaSuccess && prev != dev) err = cudaSetDevice(dev);
+    if (err == cudaSuccess) err = cudaSetDevice(dev);
     ok = (err == cudaSuccess);
   }
   ~DeviceGuard() { int cur = -1; if (cudaGetDevice(&cur) == cudaSuccess && cur != prev && prev >= 0) cudaSetDevice(prev); }
