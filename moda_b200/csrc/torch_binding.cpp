@@ -242,8 +242,15 @@ bool wants_grad(std::initializer_list<const Tensor*> xs) {
   return false;
 }
 
+// There is no forward-mode derivative: a dual number's tangent must not be dropped in silence.
+void refuse_tangents(std::initializer_list<const Tensor*> xs) {
+  for (const Tensor* x : xs)
+    TORCH_CHECK_NOT_IMPLEMENTED(!x->defined() || !x->_fw_grad(0).defined(), "moda_b200: forward-mode differentiation is not implemented");
+}
+
 Out attention(const Op& op, const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& ck, const Tensor& cv,
               const CacheStatePtr& state, const Tensor& token) {
+  refuse_tangents({&q, &k, &v, &ck, &cv});
   const bool grad = wants_grad({&q, &k, &v, state ? &token : &ck, state ? &token : &cv});
   Out r;
   {
@@ -428,6 +435,7 @@ PyObject* py_cache_append(PyObject*, PyObject* const* a, Py_ssize_t n) {
   Tensor next;
   {
     NoGil no_gil;
+    refuse_tangents({&k, &v});
     const bool grad = wants_grad({&k, &v, &token});
     moda_problem pr;
     {
