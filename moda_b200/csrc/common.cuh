@@ -55,12 +55,14 @@ __host__ __device__ __forceinline__ int64_t dep_mem_row(const Params& p, int64_t
 // and the causal imbalance between tiles is what matters: `rank` then runs over the tiles of
 // every head alike, so that the heaviest tiles of ALL heads start first and the light ones fill
 // the tail of a short launch.  (Depth rows are read once, by one block: they do not count.)
+// `parts`: neighbours in x that share a tile (a thread-block cluster).
 struct BlockId { int rank, h, b; };
-__device__ __forceinline__ BlockId block_order(const Params& p, int head_dim) {
+__device__ __forceinline__ BlockId block_order(const Params& p, int head_dim, int parts = 1) {
   const int64_t seq_kv_bytes = (int64_t)p.B * p.H * p.T_kv * head_dim * 4;     // K and V, 16-bit
-  if (seq_kv_bytes > ((int64_t)48 << 20)) return {(int)blockIdx.x, (int)blockIdx.y, (int)blockIdx.z};
+  const int bx = (int)blockIdx.x / parts, nx = (int)gridDim.x / parts;
+  if (seq_kv_bytes > ((int64_t)48 << 20)) return {bx, (int)blockIdx.y, (int)blockIdx.z};
   const int hb = (int)(gridDim.y * gridDim.z);
-  const int lin = (int)(blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * blockIdx.z));
+  const int lin = bx + nx * (int)(blockIdx.y + gridDim.y * blockIdx.z);
   const int r = lin / hb, w = lin - r * hb;
   return {r, w % (int)gridDim.y, w / (int)gridDim.y};
 }

@@ -124,6 +124,23 @@ __global__ void __launch_bounds__(256) pre_kernel(const __grid_constant__ Params
   }
 }
 
+// Thread-block clusters: rank and size, barrier over all threads (a thread that has exited is not waited
+// for), and stores into the shared memory of another CTA of the cluster.
+__device__ __forceinline__ uint32_t cluster_rank() { uint32_t r; asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r)); return r; }
+__device__ __forceinline__ uint32_t cluster_size() { uint32_t r; asm volatile("mov.u32 %0, %%cluster_nctarank;" : "=r"(r)); return r; }
+__device__ __forceinline__ void cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
+}
+__device__ __forceinline__ uint32_t cluster_addr(uint32_t smem, uint32_t rank) {
+  uint32_t r;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(smem), "r"(rank));
+  return r;
+}
+__device__ __forceinline__ void st_cluster(uint32_t addr, uint32_t x) { asm volatile("st.shared::cluster.u32 [%0], %1;" :: "r"(addr), "r"(x) : "memory"); }
+__device__ __forceinline__ void st_cluster_v4(uint32_t addr, const uint4& x) {
+  asm volatile("st.shared::cluster.v4.u32 [%0], {%1, %2, %3, %4};" :: "r"(addr), "r"(x.x), "r"(x.y), "r"(x.z), "r"(x.w) : "memory");
+}
+
 // Control block shared by both kernels (placed after the tiles):
 //   [0, 8*kMaxBars) mbarriers; then the TMEM base slot, the abort flag and the drain flag.
 constexpr int kMaxBars = 24;
@@ -512,7 +529,12 @@ constexpr uint32_t kDkvPairBytes = 2 * kScoreTile;   // P^T tile + dS^T tile
 // ([192, 256) and [320, 384): P^T in the first 32 columns of a pair, dS^T in the next 32)
 constexpr uint32_t kDkvPairCol0 = 192, kDkvPairColStride = 128;
 
-template <typename T, int D>
+// kSplit: the CTAs of a cluster share a key tile and divide its query steps (dkv_parts says when).  Each
+// accumulates its share; in the end a CTA owns a slice of the dV and dK columns, receives that
+// slice of the others' accumulators in its own shared memory (the ring is free by then) and stores
+// the sum, taken in the order of the cluster's ranks.  Every thread of every CTA reaches both cluster
+// barriers, also after a failed wait, so that no CTA is written to after it has left.
+template <typename T, int D, bool kSplit>
 __global__ void __launch_bounds__(kDkvThreads, 1)
 dkv_kernel(const __grid_constant__ Params p, const __grid_constant__ DkvMaps maps, const float* delta_t,
            const float* lse_t, int T_qp, int n_seq_key_tiles) {
@@ -536,11 +558,13 @@ dkv_kernel(const __grid_constant__ Params p, const __grid_constant__ DkvMaps map
   volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(gctl + 8 * kMaxBars);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(gctl + 8 * kMaxBars + 4);
   volatile int* drain_flag = reinterpret_cast<volatile int*>(gctl + 8 * kMaxBars + 8);
+  volatile int* peer_failed = reinterpret_cast<volatile int*>(gctl + 8 * kMaxBars + 12);
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  if (launch_failed(p)) return;
+  if (!kSplit && launch_failed(p)) return;              // (a cluster stays together: below)
+  const int parts = kSplit ? (int)cluster_size() : 1, part = kSplit ? (int)cluster_rank() : 0;
 
-  const BlockId bid = block_order(p, D);
+  const BlockId bid = block_order(p, D, parts);
   const int h = bid.h, b = bid.b;
   const bool is_dep = bid.rank >= n_seq_key_tiles;
   const int c0 = (is_dep ? bid.rank - n_seq_key_tiles : bid.rank) * kBN;
@@ -559,7 +583,12 @@ dkv_kernel(const __grid_constant__ Params p, const __grid_constant__ DkvMaps map
     q_end = t_end * p.G;
   }
   q_begin = (q_begin / kStep) * kStep;
-  const int n = (q_end - q_begin + kStep - 1) / kStep;
+  int n = (q_end - q_begin + kStep - 1) / kStep;
+  if (kSplit) {
+    const int first = n * part / parts;
+    q_begin += first * kStep;
+    n = n * (part + 1) / parts - first;
+  }
 
   if (tid == 0) {
     mbar_init(bars + 8 * B_.res, 256);
@@ -571,8 +600,9 @@ dkv_kernel(const __grid_constant__ Params p, const __grid_constant__ DkvMaps map
       mbar_init(bars + 8 * (B_.p0 + i), 128);
       mbar_init(bars + 8 * (B_.r0 + i), 128); mbar_init(bars + 8 * (B_.t0 + i), 1);
     }
-    *abort_flag = 0;
+    *abort_flag = kSplit && launch_failed(p) ? 1 : 0;
     *drain_flag = 0;
+    if (kSplit) *peer_failed = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   }
@@ -800,7 +830,7 @@ dkv_kernel(const __grid_constant__ Params p, const __grid_constant__ DkvMaps map
       // the teardown path)
     }
     if (ok && n > 0) ok = __all_sync(0xffffffffu, mbar_wait(bars + 8 * B_.done, 0, abort_flag, B_.done));
-    if (ok && n > 0) {
+    if (!kSplit && ok && n > 0) {
       tc_fence_after();
       const View& ov = (wg == 0) ? (is_dep ? p.dvd : p.dv) : (is_dep ? p.dkd : p.dk);
       T* gout = reinterpret_cast<T*>(ov.ptr) + ov.off(b, is_dep ? dep_mem_row(p, key) : (int64_t)key, h);
@@ -823,6 +853,62 @@ dkv_kernel(const __grid_constant__ Params p, const __grid_constant__ DkvMaps map
             uint4* dst = reinterpret_cast<uint4*>(gout + q4 * 32 + i * 8);
             *dst = acc ? pack8_blend<T>(ov32 + i * 8, mul, *dst, 1.f) : v4;
           }
+        }
+      }
+    }
+  }
+  if constexpr (kSplit) {
+    const int wg = warp >> 2, row = (warp & 3) * 32 + lane, key = c0 + row;      // as in the main loop
+    const int cols = D / parts;                         // of dV and of dK, owned by each CTA of the cluster
+    const uint32_t tsrc = ((wg == 0) ? tmem_dV : tmem_dK) + ((uint32_t)((warp & 3) * 32) << 16);
+    // received: [other rank][dV, dK][column quad][key row], 16 bytes each
+    const uint32_t quads = cols / 4, slot_bytes = 2 * quads * 128 * 16;
+    tc_fence_before();
+    cluster_sync();                                     // every ring of the cluster is free
+    tc_fence_after();
+    if (warp < 8) {
+      const bool mine_ok = *abort_flag == 0;
+      for (int o = 0; o < parts; ++o) {
+        if (o == part) continue;
+        const uint32_t dst = cluster_addr(sRing, o) + (part - (part > o)) * slot_bytes + (wg * quads * 128 + row) * 16;
+        if (!mine_ok) {
+          if (tid == 0) st_cluster(cluster_addr(smem_u32(const_cast<int*>(peer_failed)), o), 1u);
+          continue;
+        }
+        for (int c = 0; c < cols; c += 16) {
+          uint32_t x[16];
+          if (n > 0) { tmem_ld16(tsrc + o * cols + c, x); tmem_wait_ld(); }
+#pragma unroll
+          for (int i = 0; i < 4; ++i)
+            st_cluster_v4(dst + (c / 4 + i) * (128 * 16), n > 0 ? make_uint4(x[4 * i], x[4 * i + 1], x[4 * i + 2], x[4 * i + 3]) : make_uint4(0, 0, 0, 0));
+        }
+      }
+    }
+    cluster_sync();                                     // every slice has arrived
+    if (warp < 8 && *abort_flag == 0 && *peer_failed == 0) {
+      const View& ov = (wg == 0) ? p.dv : p.dk;         // (depth tiles are not split)
+      T* gout = reinterpret_cast<T*>(ov.ptr) + ov.off(b, key, h) + part * cols;
+      const float mul = (wg == 0) ? 1.f : p.scale;
+      const unsigned char* in = smem_raw + (wg * quads * 128 + row) * 16;
+      for (int c = 0; c < cols; c += 16) {
+        uint32_t x[16];
+        if (n > 0) { tmem_ld16(tsrc + part * cols + c, x); tmem_wait_ld(); }
+        float own[16], sum[16];
+#pragma unroll
+        for (int i = 0; i < 16; ++i) { own[i] = n > 0 ? __uint_as_float(x[i]) : 0.f; sum[i] = 0.f; }
+        for (int o = 0; o < parts; ++o) {
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            float4 f = make_float4(own[4 * i], own[4 * i + 1], own[4 * i + 2], own[4 * i + 3]);
+            if (o != part) f = *reinterpret_cast<const float4*>(in + (o - (o > part)) * slot_bytes + (c / 4 + i) * (128 * 16));
+            sum[4 * i] += f.x; sum[4 * i + 1] += f.y; sum[4 * i + 2] += f.z; sum[4 * i + 3] += f.w;
+          }
+        }
+        if (key < n_keys) {
+#pragma unroll
+          for (int i = 0; i < 16; ++i) x[i] = __float_as_uint(sum[i]);
+          *reinterpret_cast<uint4*>(gout + c) = pack8_scaled<T>(x, mul);
+          *reinterpret_cast<uint4*>(gout + c + 8) = pack8_scaled<T>(x + 8, mul);
         }
       }
     }

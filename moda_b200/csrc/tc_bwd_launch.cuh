@@ -9,6 +9,8 @@
 // and executes the five matmuls of the backward once each; measured, it is no faster (see
 // tc_bwd_fused_kernel.cuh), which is why it is not the default.
 #pragma once
+#include <algorithm>
+
 #include "tc_bwd_fused_kernel.cuh"
 
 namespace moda {
@@ -47,6 +49,26 @@ inline size_t bwd_extra_workspace_bytes(const moda_problem* pr) { return BwdWork
 
 struct BwdMaps { DqMaps dq; DkvMaps dkv; DgOutMaps out; };
 struct BwdBuffers { float *delta_t, *lse_t, *norm_t; float4* scale_blk; int* kvmax; int* dq_acc; size_t acc_bytes, kvmax_bytes; };
+
+// CTAs that share a key tile of the dk/dv kernel.  A tile's query steps are a serial chain on one SM and
+// under a causal mask the first tile has twice the average: with few tiles the launch lasts as long as
+// that one.  Estimate in steps of 64 query rows, per CTA kFixed more (set-up, first loads, the sums' way
+// through the cluster, the stores and the SMs that pairs leave idle): the longest CTA, or all of them
+// over the SMs; a split has to win a tenth.  D = 128: B = 2, T = 2048, H = 4, G = 4 (128 tiles): two CTAs 116 -> 81 us;
+// B = 3, T = 1531, H = 5, G = 2 (180 tiles): two CTAs 67 -> 85 us, so one; kFixed = 20 puts both right.
+inline int dkv_parts(const Params& p, int n_sm) {
+  constexpr double kFixed = 20;
+  const double tiles = (double)((p.T_kv + kBN - 1) / kBN) * p.H * p.B;
+  const double longest = (p.T_q + kStep - 1) / kStep, all = tiles * longest * (p.mode == kNonCausal ? 1.0 : 0.5);
+  double best = std::max(longest + kFixed, (all + tiles * kFixed) / n_sm);
+  int parts = 1;
+  for (int n = 2; n <= 4; n *= 2) {
+    if (longest < 2 * n) break;
+    const double t = std::max(longest / n + kFixed, (all + n * tiles * kFixed) / n_sm);
+    if (t < 0.9 * best) { best = t; parts = n; }
+  }
+  return parts;
+}
 
 template <typename T, int D>
 inline cudaError_t launch_bwd(const Params& p, const BwdMaps& m, const BwdBuffers& w, int T_qp, bool dg, bool fused,
@@ -108,7 +130,7 @@ inline cudaError_t launch_bwd(const Params& p, const BwdMaps& m, const BwdBuffer
       if ((e = cudaGetLastError()) != cudaSuccess) return e;
       *launches += 1;
       if (!dg && n_dep_tiles > 0) {   // depth key tiles the query-stationary kernel cannot own: key-parallel kernel on them alone
-        auto kern = dkv_kernel<T, D>;
+        auto kern = dkv_kernel<T, D, false>;
         if ((e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dkv_smem)) != cudaSuccess) return e;
         dim3 grid(n_dep_tiles, p.H, p.B);
         prof::Scope ps(prof::kDkvTc, st);
@@ -128,13 +150,25 @@ inline cudaError_t launch_bwd(const Params& p, const BwdMaps& m, const BwdBuffer
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
     *launches += 1;
     {
-      auto kern = dkv_kernel<T, D>;
+      const bool own_tiles = !dg && n_dep_tiles > 0;
+      const int parts = own_tiles ? 1 : dkv_parts(p, n_sm);
+      auto kern = parts > 1 ? dkv_kernel<T, D, true> : dkv_kernel<T, D, false>;
       if ((e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dkv_smem)) != cudaSuccess) return e;
-      dim3 grid(n_seq + (dg ? 0 : n_dep_tiles), p.H, p.B);
+      cudaLaunchConfig_t cfg{};
+      cfg.gridDim = dim3((n_seq + (own_tiles ? n_dep_tiles : 0)) * parts, p.H, p.B);
+      cfg.blockDim = dim3(kDkvThreads);
+      cfg.dynamicSmemBytes = dkv_smem;
+      cfg.stream = st;
+      cudaLaunchAttribute cluster{};
+      cluster.id = cudaLaunchAttributeClusterDimension;
+      cluster.val.clusterDim.x = parts;
+      cluster.val.clusterDim.y = cluster.val.clusterDim.z = 1;
+      cfg.attrs = &cluster;
+      cfg.numAttrs = parts > 1 ? 1 : 0;
       prof::Scope ps(prof::kDkvTc, st);
-      kern<<<grid, kDkvThreads, dkv_smem, st>>>(p, m.dkv, delta_t, lse_t, T_qp, n_seq);
+      e = cudaLaunchKernelEx(&cfg, kern, p, m.dkv, (const float*)delta_t, (const float*)lse_t, T_qp, n_seq);
     }
-    if ((e = cudaGetLastError()) != cudaSuccess) return e;
+    if (e != cudaSuccess) return e;
     *launches += 1;
   }
   if (dg) {
