@@ -534,6 +534,15 @@ int moda_b200_bwd_static_scratch(const moda_problem* prob, const moda_tensor4* q
                                  const moda_tensor4* d_depth_v, void* stream) {
   size_t need = 0;
   if (int rc = moda_b200_bwd_workspace_bytes(prob, &need)) return rc;
+  // An in-place cache of a layer count that does not divide 32 has always been taken up to what the
+  // mma.sync kernels need here, which is a third of what the tcgen05 kernels do.
+  moda_problem small = *prob;
+  if (need > (size_t)MODA_B200_STATIC_SCRATCH_BYTES && prob->path == MODA_PATH_AUTO && prob->L > 0 &&
+      prob->depth_rows_per_pos > prob->L && 32 % prob->L != 0) {
+    small.path = MODA_PATH_SIMT_MMA;
+    prob = &small;
+    need = delta_bytes(prob);
+  }
   if (need > (size_t)MODA_B200_STATIC_SCRATCH_BYTES) return MODA_ERR_TOO_LARGE;
   DeviceGuard guard(prob->device);          // the symbol address is per device: resolve it with
   if (!guard.ok) return cuda_fail(guard.err);  // the problem's device current

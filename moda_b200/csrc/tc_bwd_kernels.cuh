@@ -219,6 +219,7 @@ dq_kernel(const __grid_constant__ Params p, const __grid_constant__ DqMaps maps,
   const int h = bid.h, b = bid.b;
   const int r0 = qt * kBM;
   int n_seq, n_dep, dep_c0, seq_full_hi;   // key walk in steps of 64
+  const int dep_rows = dep_tile_rows(p, kStep);
   {
     const int r_last = min(r0 + kBM, p.T_q) - 1;
     int lo, hi, lo2, hi2;
@@ -229,7 +230,7 @@ dq_kernel(const __grid_constant__ Params p, const __grid_constant__ DqMaps maps,
     dep_interval(p, r0, lo, hi);
     dep_interval(p, r_last, lo2, hi2);
     dep_c0 = lo;
-    n_dep = (hi2 - lo + kStep - 1) / kStep;
+    n_dep = (hi2 - lo + dep_rows - 1) / dep_rows;
   }
   // dq_acc != nullptr: the sequence keys' share of dQ is already in the fixed-point accumulator the
   // fused key-stationary kernel filled (tc_bwd_fused_kernel.cuh); this kernel then walks the depth
@@ -253,6 +254,7 @@ dq_kernel(const __grid_constant__ Params p, const __grid_constant__ DqMaps maps,
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   }
+  if (n_dep > 0 && dep_rows < kStep) zero_tails(smem_raw, R * 2 * (D / 64), kStep, dep_rows);
   if (warp == 0) {
     tmem_alloc(bars + 8 * kMaxBars, 512);
     tmem_relinquish();
@@ -274,12 +276,12 @@ dq_kernel(const __grid_constant__ Params p, const __grid_constant__ DqMaps maps,
         const uint32_t slot = i % R;
         if (i >= R && !(ok = mbar_wait(bars + 8 * (B_.empty0 + slot), ((i / R) - 1) & 1, abort_flag, B_.empty0 + slot))) break;
         const bool dep = i >= n_seq;
-        const int row = dep ? dep_c0 + (i - n_seq) * kStep : i * kStep;
+        const int row = dep ? dep_c0 + (i - n_seq) * dep_rows : i * kStep;
         const uint32_t dst = sRing + slot * 2 * kStepTile, bar = bars + 8 * (B_.full0 + slot);
         const CUtensorMap* mk = dep ? &maps.kd : &maps.k;
         const CUtensorMap* mv = dep ? &maps.vd : &maps.v;
         if (elect_one()) {
-          mbar_expect_tx(bar, 2 * kStepTile);
+          mbar_expect_tx(bar, dep ? 2 * dep_rows * 2 * D : 2 * kStepTile);
           if (dep) {
             tma_load_dep_tile<D>(dst, mk, bar, kStepHalf, h, row, b, dep5);
             tma_load_dep_tile<D>(dst + kStepTile, mv, bar, kStepHalf, h, row, b, dep5);
@@ -407,9 +409,9 @@ dq_kernel(const __grid_constant__ Params p, const __grid_constant__ DqMaps maps,
       if (!ok) break;
       tc_fence_after();
       const bool is_dep = i >= n_seq;
-      const int c0 = is_dep ? dep_c0 + (i - n_seq) * kStep : i * kStep;
+      const int c0 = is_dep ? dep_c0 + (i - n_seq) * dep_rows : i * kStep;
       const bool masked = is_dep || (c0 + kStep > seq_full_hi);
-      const int lo = is_dep ? dlo : slo, hi = is_dep ? dhi : shi;
+      const int lo = is_dep ? dlo : slo, hi = is_dep ? min(dhi, c0 + dep_rows) : shi;
       const uint32_t tS = tmem + (i & 1) * 128 + lane_addr;
       uint32_t su[64], du[64];
       tmem_ld32<0>(tS, su);
@@ -962,7 +964,7 @@ struct DgOutMaps { CUtensorMap dkd, dvd; };                                     
 constexpr int kDgThreads = 320;                                                 // 8 softmax/store warps, MMA warp, TMA warp
 
 // One 64-row query block of the depth-gradient kernel.
-struct DgBlock { int q0, h, b, k_lo, k_hi, n; int64_t stat_base; };
+struct DgBlock { int q0, h, b, k_lo, k_hi, n, rows; int64_t stat_base; };
 __device__ __forceinline__ DgBlock dg_block(const Params& p, int idx, int n_xb, int T_qp) {
   DgBlock k;
   const int xb = idx % n_xb, hb = idx / n_xb;
@@ -973,7 +975,8 @@ __device__ __forceinline__ DgBlock dg_block(const Params& p, int idx, int n_xb, 
   int tmp;
   dep_interval(p, k.q0, k.k_lo, tmp);
   dep_interval(p, r_last, tmp, k.k_hi);
-  k.n = (k.k_hi - k.k_lo + kBN - 1) / kBN;              // key tiles of 128
+  k.rows = dep_tile_rows(p, kBN);
+  k.n = (k.k_hi - k.k_lo + k.rows - 1) / k.rows;        // key tiles of 128
   k.stat_base = ((int64_t)k.b * p.H + k.h) * T_qp;
   return k;
 }
@@ -1049,10 +1052,10 @@ depth_grad_kernel(const __grid_constant__ Params p, const __grid_constant__ DkvM
         const int gi = g + i;
         const uint32_t slot = gi & 1;
         if (gi >= 2 && !mbar_wait(bars + 8 * (kDgEmpty0 + slot), ((gi >> 1) - 1) & 1, abort_flag, kDgEmpty0 + slot)) return false;
-        const int row = k.k_lo + i * kBN;
+        const int row = k.k_lo + i * k.rows;
         const uint32_t dst = sKV + slot * 2 * kTile, bar = bars + 8 * (kDgFull0 + slot);
         if (elect_one()) {
-          mbar_expect_tx(bar, 2 * kTile);
+          mbar_expect_tx(bar, 2 * k.rows * 2 * D);
           tma_load_dep_tile<D>(dst, &maps.kd, bar, kHalfBytes, k.h, row, k.b, dep5);
           tma_load_dep_tile<D>(dst + kTile, &maps.vd, bar, kHalfBytes, k.h, row, k.b, dep5);
         }
@@ -1146,6 +1149,7 @@ depth_grad_kernel(const __grid_constant__ Params p, const __grid_constant__ DkvM
     const int row = wq * 32 + lane;                   // key row of the tile == TMEM lane
     const uint32_t lane_addr = (uint32_t)(wq * 32) << 16;
     const float c = p.scale_log2;
+    const bool boxes = dep5 == 0 || 32 % dep5 == 0;   // 32 rows are whole positions: they can leave as a box
     bool ok = true;
     int g = 0, kb = 0;
     for (int idx = blockIdx.x; ok && idx < total; idx += gridDim.x) {
@@ -1156,9 +1160,9 @@ depth_grad_kernel(const __grid_constant__ Params p, const __grid_constant__ DkvM
       // over its scores
       auto softmax = [&](int i) -> bool {
         const int gj = g + i;
-        const int key = k.k_lo + i * kBN + row;
+        const int key = k.k_lo + i * k.rows + row;
         int jlo = 0, jn = 0;                            // query rows [q0 + jlo, q0 + jlo + jn) see this key
-        if (key < k.k_hi) {
+        if (row < k.rows && key < k.k_hi) {
           const int tp = key / p.L;
           const int rlo = tp * p.G;
           const int rhi = ((p.mode == kChunkVisible) ? min((tp / p.Cb + 1) * p.Cb, p.T_kv) : tp + 1) * p.G;
@@ -1211,10 +1215,10 @@ depth_grad_kernel(const __grid_constant__ Params p, const __grid_constant__ DkvM
         ok = __all_sync(0xffffffffu, mbar_wait(bars + 8 * kDgU, (g + i) & 1, abort_flag, kDgU));
         if (!ok) break;
         tc_fence_after();
-        const int key0 = k.k_lo + i * kBN + wq * 32;         // first key row of this warp
+        const int key0 = k.k_lo + i * k.rows + wq * 32;      // first key row of this warp
         const uint32_t tacc = (wg ? tmem_dK : tmem_dV) + lane_addr;
         const float f = wg ? p.scale : 1.f;
-        if (key0 + 32 <= k.k_hi && !p.acc_depth) {           // every row of the warp is this block's
+        if (key0 + 32 <= k.k_hi && !p.acc_depth && boxes) {  // every row of the warp is this block's
           if (lane == 0) bulk_wait_read_all();               // this warp's previous store has read its rows
           __syncwarp();
           // staging = the TMA box layout: two [128 rows x 128 B] halves per tensor, 16-byte chunk c of
@@ -1248,7 +1252,7 @@ depth_grad_kernel(const __grid_constant__ Params p, const __grid_constant__ DkvM
           __syncwarp();
         } else {
           const int key = key0 + lane;
-          const bool valid = key < k.k_hi;
+          const bool valid = key < min(k.k_hi, k.k_lo + (i + 1) * k.rows);
           const int64_t mrow = dep_mem_row(p, valid ? key : k.k_lo);
           T* gout = wg ? reinterpret_cast<T*>(p.dkd.ptr) + p.dkd.off(k.b, mrow, k.h) : reinterpret_cast<T*>(p.dvd.ptr) + p.dvd.off(k.b, mrow, k.h);
 #pragma unroll

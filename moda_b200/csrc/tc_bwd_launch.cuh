@@ -222,7 +222,8 @@ inline int bwd(const Params& p, const moda_problem* pr, void* extra, int n_sm, c
   }
   if (!ok) return MODA_ERR_UNSUPPORTED;
   const bool dg = depth_grad_applies(p, pr);
-  if (dg && !(make_map_depth(&m.out.dkd, p.dkd, dt, p, D, 32) && make_map_depth(&m.out.dvd, p.dvd, dt, p, D, 32)))
+  const bool boxes = p.Ls == p.L || (dep && 32 % p.L == 0);      // depth_grad_kernel stores boxes of 32 rows, or row by row
+  if (dg && boxes && !(make_map_depth(&m.out.dkd, p.dkd, dt, p, D, 32) && make_map_depth(&m.out.dvd, p.dvd, dt, p, D, 32)))
     return MODA_ERR_UNSUPPORTED;
   if ((int64_t)((p.T_q + kStep - 1) / kStep) * p.H * p.B > 0x7fffffff || n_sm <= 0) return MODA_ERR_UNSUPPORTED;
 

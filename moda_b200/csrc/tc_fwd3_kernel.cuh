@@ -61,12 +61,14 @@ struct F3Plan {
   Walk w[2];
   int n_s;      // sequence steps
   int n;        // all steps
+  int dep_rows; // depth rows of a depth tile
 };
 __device__ __forceinline__ F3Plan f3_plan(const Params& p, int r0) {
   F3Plan pl;
   pl.w[0] = make_walk(p, r0);
   if (r0 + kBM < p.T_q) pl.w[1] = make_walk(p, r0 + kBM);
   else { pl.w[1].n_seq = 0; pl.w[1].n_dep = 0; pl.w[1].dep_c0 = 0; pl.w[1].seq_full_hi = 0; }
+  pl.dep_rows = dep_tile_rows(p, kBN);
   pl.n_s = max(pl.w[0].n_seq, pl.w[1].n_seq);
   pl.n = pl.n_s + pl.w[0].n_dep + pl.w[1].n_dep;
   return pl;
@@ -85,7 +87,7 @@ __device__ __forceinline__ void f3_step(const F3Plan& pl, int s, int& part, bool
   else { a = (pl.w[0].n_dep > pl.w[1].n_dep) ? 0 : 1; d = m + (e - 2 * m); }
   part = 1 << a;
   is_dep = true;
-  row = pl.w[a].dep_c0 + d * kBN;
+  row = pl.w[a].dep_c0 + d * pl.dep_rows;
 }
 
 // 16 columns of pk starting at column j (j is a compile-time constant after unrolling)
@@ -169,6 +171,7 @@ fwd3_kernel(const __grid_constant__ Params p, const __grid_constant__ Fwd3Maps m
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   }
+  if (pl.n > pl.n_s && pl.dep_rows < kBN) zero_tails(smem_raw + (2 + KS) * kTile, 2 * (D / 64), kBN, pl.dep_rows);   // V
   if (warp == 0) {
     tmem_alloc(bars + 8 * kMaxBars, 512);
     tmem_relinquish();
@@ -207,7 +210,7 @@ fwd3_kernel(const __grid_constant__ Params p, const __grid_constant__ Fwd3Maps m
         const uint32_t dst = is_k ? sK + slot * kTile : sV + slot * kTile, bar = bars + 8 * f_bar;
         const CUtensorMap* m = dep ? (is_k ? &maps.kd : &maps.vd) : (is_k ? &maps.k : &maps.v);
         if (elect_one()) {
-          mbar_expect_tx(bar, kTile);
+          mbar_expect_tx(bar, dep ? pl.dep_rows * 2 * D : kTile);
           if (dep) tma_load_dep_tile<D>(dst, m, bar, kHalfBytes, h, row, b, dep5);
           else tma_load_tile<D>(dst, m, bar, kHalfBytes, h, row, b);
         }
@@ -387,11 +390,11 @@ fwd3_kernel(const __grid_constant__ Params p, const __grid_constant__ Fwd3Maps m
       if (!ok) break;   // warp-uniform: the tcgen05 loads/stores below are warp-collective
       tc_fence_after();
       const bool masked = is_dep || (c0 + kBN > walk.seq_full_hi);
-      const int lo = is_dep ? dlo : slo, hi = is_dep ? dhi : shi;
+      const int lo = is_dep ? dlo : slo, hi = is_dep ? min(dhi, c0 + pl.dep_rows) : shi;
 
       // A depth tile holds the rows of several positions; a warp whose 32 query rows see none of
       // its columns contributes an all-zero P block and skips the scores altogether.
-      const bool none = is_dep && __all_sync(0xffffffffu, (c0 + kBN <= lo) || (c0 >= hi));
+      const bool none = is_dep && __all_sync(0xffffffffu, (c0 + pl.dep_rows <= lo) || (c0 >= hi));
       // P is complete for a group of columns once every lane's stores have finished: one arrival per warp
       auto p_ready = [&](int bar_id) {
         tmem_wait_st();

@@ -354,6 +354,21 @@ __host__ __device__ constexpr uint32_t instr_desc(uint32_t fmt, uint32_t n, bool
 
 enum BarId : int { kBarQ = 0, kBarK, kBarV, kBarS, kBarP, kBarO, kBarKFree, kBarVFree, kBarCount };
 
+// Depth rows that a tile of `rows` key rows holds: all of them, except for an in-place layer cache, whose
+// TMA boxes are whole positions of L rows.  What a box leaves of the tile is zeros (zero_tails) or
+// stale rows of sequence keys, and its columns are masked.
+__host__ __device__ __forceinline__ int dep_tile_rows(const Params& p, int rows) {
+  return (p.Ls == p.L) ? rows : rows / p.L * p.L;
+}
+// Zeros in the rows [used, rows) of n_boxes consecutive boxes of `rows` rows of 128 bytes: what no box
+// of depth rows fills must not hold an earlier kernel's bytes, since 0 x NaN is NaN in a matmul.
+__device__ __forceinline__ void zero_tails(unsigned char* boxes, int n_boxes, int rows, int used) {
+  const int per = (rows - used) * 8;
+  for (int i = threadIdx.x; i < n_boxes * per; i += blockDim.x)
+    *reinterpret_cast<uint4*>(boxes + ((i / per) * rows + used) * 128 + (i % per) * 16) = make_uint4(0, 0, 0, 0);
+  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+}
+
 // Tile walk of a 128-row query tile (same construction as simt::make_walk).
 struct Walk { int n_seq, n_dep, dep_c0, seq_full_hi; };
 __device__ __forceinline__ Walk make_walk(const Params& p, int r0) {
@@ -367,7 +382,8 @@ __device__ __forceinline__ Walk make_walk(const Params& p, int r0) {
   dep_interval(p, r0, lo, hi);
   dep_interval(p, r_last, lo2, hi2);
   w.dep_c0 = lo;
-  w.n_dep = (hi2 - lo + kBN - 1) / kBN;
+  const int dep_rows = dep_tile_rows(p, kBN);
+  w.n_dep = (hi2 - lo + dep_rows - 1) / dep_rows;
   return w;
 }
 
@@ -420,7 +436,7 @@ fwd_kernel(const __grid_constant__ Params p, const __grid_constant__ FwdMaps map
   const int h = bid.h, b = bid.b;
   const int r0 = qt * kBM;
   const Walk walk = make_walk(p, r0);
-  const int n_tiles = walk.n_seq + walk.n_dep;
+  const int n_tiles = walk.n_seq + walk.n_dep, dep_rows = dep_tile_rows(p, kBN);
   const int dep5 = (p.Ls != p.L) ? p.L : 0;      // in-place layer cache: 5-D depth maps
 
   if (tid == 0) {
@@ -437,6 +453,7 @@ fwd_kernel(const __grid_constant__ Params p, const __grid_constant__ FwdMaps map
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   }
+  if (walk.n_dep > 0 && dep_rows < kBN) zero_tails(gbase + 2 * kTile, D / 64, kBN, dep_rows);   // V
   if (warp == 0) {
     tmem_alloc(ctl + 64, 256);
     tmem_relinquish();
@@ -457,12 +474,12 @@ fwd_kernel(const __grid_constant__ Params p, const __grid_constant__ FwdMaps map
       uint32_t pend_k_par = 0, pend_v_par = 0;
       auto load_kv = [&](int i, bool is_k) {
         const bool dep = i >= walk.n_seq;
-        const int row = dep ? walk.dep_c0 + (i - walk.n_seq) * kBN : i * kBN;
+        const int row = dep ? walk.dep_c0 + (i - walk.n_seq) * dep_rows : i * kBN;
         const CUtensorMap* m = is_k ? (dep ? &maps.kd : &maps.k) : (dep ? &maps.vd : &maps.v);
         const uint32_t dst = is_k ? sK : sV;
         const uint32_t bar = bars + 8 * (is_k ? kBarK : kBarV);
         if (elect_one()) {
-          mbar_expect_tx(bar, kTile);
+          mbar_expect_tx(bar, dep ? dep_rows * 2 * D : kTile);
           if (dep) tma_load_dep_tile<D>(dst, m, bar, kHalfBytes, h, row, b, dep5);
           else tma_load_tile<D>(dst, m, bar, kHalfBytes, h, row, b);
         }
@@ -543,13 +560,13 @@ fwd_kernel(const __grid_constant__ Params p, const __grid_constant__ FwdMaps map
       if (!ok) break;   // warp-uniform: the tcgen05 loads/stores below are warp-collective
       tc_fence_after();
       const bool is_dep = j >= walk.n_seq;
-      const int c0 = is_dep ? walk.dep_c0 + (j - walk.n_seq) * kBN : j * kBN;
+      const int c0 = is_dep ? walk.dep_c0 + (j - walk.n_seq) * dep_rows : j * kBN;
       const bool masked = is_dep || (c0 + kBN > walk.seq_full_hi);
-      const int lo = is_dep ? dlo : slo, hi = is_dep ? dhi : shi;
+      const int lo = is_dep ? dlo : slo, hi = is_dep ? min(dhi, c0 + dep_rows) : shi;
 
       // A depth tile holds the rows of several positions; a warp whose 32 query rows see none of
       // its columns contributes an all-zero P block and skips the scores altogether.
-      const bool none = is_dep && __all_sync(0xffffffffu, (c0 + kBN <= lo) || (c0 >= hi));
+      const bool none = is_dep && __all_sync(0xffffffffu, (c0 + dep_rows <= lo) || (c0 >= hi));
       float alpha = 1.f;
       bool grow = false;
       uint32_t pk[64];
@@ -665,11 +682,11 @@ inline bool make_map_rows(CUtensorMap* m, const View& v, int dtype, int B, int64
 }
 
 // Depth K/V (or their gradients) of an in-place layer cache: rows (t, l), l < L, at memory row
-// t * Ls + l.  5-D map (D, H, L, T, B), box [64, 1, L, box_rows / L, 1]: a tile of box_rows
-// consecutive depth rows of the operator.  box_rows must be a multiple of L.
+// t * Ls + l.  5-D map (D, H, L, T, B), box [64, 1, L, box_rows / L, 1]: a tile of as many whole
+// positions as box_rows holds (dep_tile_rows).
 inline bool make_map_dep5(CUtensorMap* m, const View& v, int dtype, int B, int T, int L, int Ls, int H, int D, int box_rows) {
   EncodeTiledFn fn = encode_fn();
-  if (fn == nullptr || v.ptr == nullptr || L <= 0 || box_rows % L != 0) return false;
+  if (fn == nullptr || v.ptr == nullptr || L <= 0 || box_rows < L) return false;
   if ((H > 1 && v.sh <= 0) || v.st <= 0 || (B > 1 && v.sb <= 0)) return false;
   cuuint64_t dims[5] = {(cuuint64_t)D, (cuuint64_t)H, (cuuint64_t)L, (cuuint64_t)T, (cuuint64_t)B};
   cuuint64_t strides[4] = {(cuuint64_t)((H > 1 ? v.sh : 8) * 2), (cuuint64_t)(v.st * 2), (cuuint64_t)(v.st * 2 * Ls),
@@ -687,9 +704,11 @@ inline bool make_map_depth(CUtensorMap* m, const View& v, int dtype, const Param
 }
 
 // The tcgen05 kernels take a positive scale (the row maximum is taken before scaling) and, for an
-// in-place layer cache (depth_rows_per_pos > L), a layer count that divides the 32-row boxes.
+// in-place layer cache (depth_rows_per_pos > L), at most 64 layers: a position fits the step tile of the
+// smallest pipeline (dq).  A forced path keeps to layer counts that divide 32.
 inline bool depth_layout_supported(const moda_problem* pr) {
-  return pr->L == 0 || pr->depth_rows_per_pos <= pr->L || (32 % pr->L) == 0;
+  if (pr->L == 0 || pr->depth_rows_per_pos <= pr->L || (32 % pr->L) == 0) return true;
+  return pr->path == MODA_PATH_AUTO && pr->L <= 64;
 }
 inline bool fwd_supported(const moda_problem* pr) {
   return (pr->D == 128 || pr->D == 64) && pr->mode != MODA_DEPTH_ONLY && pr->scale > 0.f && depth_layout_supported(pr);
