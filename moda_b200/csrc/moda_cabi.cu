@@ -18,6 +18,7 @@
 #include "tc_fwd3_kernel.cuh"
 #include "tc_bwd_launch.cuh"
 #include "mma_rate_probe.cuh"
+#include "short_bwd_kernel.cuh"
 
 namespace {
 
@@ -268,6 +269,29 @@ int tc_forward(const Params& p, const moda_problem* prob, int n_sm, cudaStream_t
   return tc::fwd(p, prob, st, &g_last_launches, &g_last_cuda_error);
 }
 
+// Short sequences take the one-CTA-per-head backward where its kernel has a CTA for the whole problem: 256
+// keys are what 16 warps hold in registers at D = 64, and 512 query rows keep it from being longer than the
+// tile kernels, whose matrix instructions are faster (T = 197, 256 heads or more: 351 us against 404).
+bool use_short_bwd(const moda_problem* att) {
+  return att->path == MODA_PATH_AUTO && att->mode != MODA_DEPTH_ONLY && att->D == shortseq::kD && att->L == 0 &&
+         att->T_kv <= shortseq::kMaxKeys && (int64_t)att->T_kv * att->G <= 2 * shortseq::kMaxKeys &&
+         (int64_t)att->B * att->H <= 0x7fffffff;
+}
+template <typename T>
+int short_bwd(const Params& p, cudaStream_t st) {
+  auto kern = shortseq::bwd_kernel<T>;
+  const int warps = (p.T_kv + 15) / 16;
+  const size_t smem = shortseq::smem_bytes(warps);
+  if (int rc = opt_in_smem(kern, shortseq::smem_bytes(shortseq::kMaxKeys / 16))) return rc;
+  {
+    prof::Scope ps(prof::kBwdShort, st);
+    kern<<<p.B * p.H, warps * 32, smem, st>>>(p);
+  }
+  MODA_CUDA(cudaGetLastError());
+  g_last_launches += 1;
+  return MODA_OK;
+}
+
 size_t delta_bytes(const moda_problem* pr) {
   const size_t n = (size_t)pr->B * pr->T_kv * pr->G * pr->H * sizeof(float);
   return (n + 255) & ~(size_t)255;
@@ -437,6 +461,8 @@ int moda_b200_bwd(const moda_problem* prob, const moda_tensor4* q, const moda_te
     if (int rc = fda_dispatch(p, prob, true, n_sm, st)) return rc;
     p = sequence_part(p);
   }
+  if (path == MODA_PATH_TCGEN05 && use_short_bwd(&att))
+    return prob->dtype == MODA_BF16 ? short_bwd<__nv_bfloat16>(p, st) : short_bwd<__half>(p, st);
   if (path == MODA_PATH_TCGEN05) {
     void* extra = reinterpret_cast<unsigned char*>(workspace) + delta_bytes(prob);
     return tc::bwd(p, &att, extra, n_sm, st, &g_last_launches, &g_last_cuda_error);
