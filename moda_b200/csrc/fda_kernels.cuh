@@ -130,16 +130,23 @@ __device__ __forceinline__ Step first_step(const Params& p) {
 struct Maps { CUtensorMap k, v, kt, vt, q, dout, o; };
 struct OutMaps { CUtensorMap dk, dv, dkt, dvt; };     // the same boxes of the depth gradients
 
-// Shared memory of a block: per warp two stages {K tile, V tile}; per warp one group of the query rows
-// of q (NQ = 1) or q, dout, o (NQ = 3); per warp two mbarriers; the abort words.
+// Shared memory of a block: per warp two stages {K tile, V tile} (NT = 2) or {K, V, dK, dV} (NT = 4: gradients
+// that are added to); per warp one group of the query rows of q (NQ = 1) or q, dout, o (NQ = 3); per
+// warp two mbarriers; the abort words.
 template <int D> __host__ __device__ constexpr uint32_t tile_bytes() { return kRows * 2 * D; }
-template <int D, int NQ> __host__ __device__ constexpr uint32_t smem_bytes(int G) {
-  return kWarps * (4 * tile_bytes<D>() + NQ * (G < 8 ? G : 8) * 2 * D + 16) + 16;
+// Tiles of a backward stage.  Gradients to add to are in HBM like K and V, and loaded where they are
+// added they stall the warp once a step; at D = 64 they are tiles of the ring.  At D = 128 that would
+// leave one block an SM, and they are loaded row by row.  B = 64, T = 197, H = 6, D = 64: eleven calls of L = 1..11
+// layers 1.33 -> 1.02 ms, fifteen of 1..15 2.04 -> 1.56 ms.
+template <int D, bool kAdd> __host__ __device__ constexpr int bwd_tiles() { return kAdd && D == 64 ? 4 : 2; }
+template <int D, int NQ, int NT = 2> __host__ __device__ constexpr uint32_t smem_bytes(int G) {
+  return kWarps * (2 * NT * tile_bytes<D>() + NQ * (G < 8 ? G : 8) * 2 * D + 16) + 16;
 }
 
 // The ring of one warp.
-template <int D, int NQ>
+template <int D, int NQ, int NT = 2>
 struct Ring {
+  static constexpr uint32_t kStage = NT * tile_bytes<D>();
   unsigned char *tiles, *queries;
   uint32_t bars;
   volatile int* abort_flag;
@@ -147,9 +154,9 @@ struct Ring {
   __device__ __forceinline__ Ring(const Params& p, unsigned char* smem) {
     const int w = threadIdx.x >> 5;
     const uint32_t q_bytes = NQ * min(p.G, 8) * 2 * D;
-    tiles = smem + w * 4 * tile_bytes<D>();
-    queries = smem + kWarps * 4 * tile_bytes<D>() + w * q_bytes;
-    unsigned char* ctl = smem + kWarps * (4 * tile_bytes<D>() + q_bytes);
+    tiles = smem + w * 2 * kStage;
+    queries = smem + kWarps * 2 * kStage + w * q_bytes;
+    unsigned char* ctl = smem + kWarps * (2 * kStage + q_bytes);
     bars = smem_u32(ctl) + w * 16;
     abort_flag = reinterpret_cast<volatile int*>(ctl + kWarps * 16);     // abort, drain
     if (threadIdx.x == 0) abort_flag[0] = abort_flag[1] = 0;
@@ -162,14 +169,18 @@ struct Ring {
     __syncthreads();
   }
   // Loads of step s; a unit's first step brings the query rows.
-  __device__ __forceinline__ void issue(const Params& p, const Maps& maps, const Step& s) {
+  __device__ __forceinline__ void issue(const Params& p, const Maps& maps, const OutMaps* grads, const Step& s) {
     if (tc::elect_one()) {
       const int n = min(p.L - s.l0, kRows), row = s.t * p.Ls + s.l0;
-      const uint32_t bar = bars + 8 * (issued & 1), dst = smem_u32(tiles) + (issued & 1) * 2 * tile_bytes<D>();
+      const uint32_t bar = bars + 8 * (issued & 1), dst = smem_u32(tiles) + (issued & 1) * kStage;
       const uint32_t q_rows = min(p.G, 8) * 2 * D;
-      tc::mbar_expect_tx(bar, n * 4 * D + (s.l0 == 0 ? NQ * q_rows : 0));
+      tc::mbar_expect_tx(bar, n * NT * 2 * D + (s.l0 == 0 ? NQ * q_rows : 0));
       tc::tma_load_tile<D>(dst, n == kRows ? &maps.k : &maps.kt, bar, kRows * 128, s.h, row, s.b);
       tc::tma_load_tile<D>(dst + tile_bytes<D>(), n == kRows ? &maps.v : &maps.vt, bar, kRows * 128, s.h, row, s.b);
+      if constexpr (NT == 4) {
+        tc::tma_load_tile<D>(dst + 2 * tile_bytes<D>(), n == kRows ? &grads->dk : &grads->dkt, bar, kRows * 128, s.h, row, s.b);
+        tc::tma_load_tile<D>(dst + 3 * tile_bytes<D>(), n == kRows ? &grads->dv : &grads->dvt, bar, kRows * 128, s.h, row, s.b);
+      }
       if (s.l0 == 0) {
         const int r = s.t * p.G + s.g0;
         tc::tma_load_4d(smem_u32(queries), &maps.q, bar, 0, s.h, r, s.b);
@@ -195,7 +206,7 @@ struct Ring {
     __syncwarp();
     if (tc::elect_one()) {
       const bool full = p.L - s.l0 >= kRows;
-      const uint32_t src = smem_u32(tiles) + ((taken - 1) & 1) * 2 * tile_bytes<D>();
+      const uint32_t src = smem_u32(tiles) + ((taken - 1) & 1) * kStage;
       const int row = s.t * p.Ls + s.l0;
 #pragma unroll
       for (int bx = 0; bx < D / 64; ++bx) {
@@ -214,7 +225,7 @@ struct Ring {
   __device__ __forceinline__ void drain() {
     for (int i = taken - 1; i < issued; ++i) tc::mbar_wait(bars + 8 * (i & 1), (i >> 1) & 1, abort_flag + 1, 30);
   }
-  __device__ __forceinline__ const unsigned char* stage() const { return tiles + ((taken - 1) & 1) * 2 * tile_bytes<D>(); }
+  __device__ __forceinline__ const unsigned char* stage() const { return tiles + ((taken - 1) & 1) * kStage; }
 };
 template <int D> __device__ __forceinline__ uint4 query_chunk(const unsigned char* rows, int r, int c) {
   return *reinterpret_cast<const uint4*>(rows + r * 2 * D + c * 16);
@@ -247,8 +258,8 @@ __device__ __forceinline__ void add_transposed(float (&acc)[8][2], const unsigne
 
 // kOne: L <= 16, a unit is one step.  The rows of a stage that no unit fills are then zeroed once, the
 // probabilities are normalised before P V, and nothing is carried from step to step.
-template <int D, int NQ> __device__ __forceinline__ void zero_tiles(const Ring<D, NQ>& ring) {
-  for (uint32_t i = (threadIdx.x & 31) * 16; i < 4 * tile_bytes<D>(); i += 32 * 16) *reinterpret_cast<uint4*>(ring.tiles + i) = make_uint4(0, 0, 0, 0);
+template <int D, int NQ, int NT> __device__ __forceinline__ void zero_tiles(const Ring<D, NQ, NT>& ring) {
+  for (uint32_t i = (threadIdx.x & 31) * 16; i < 2 * ring.kStage; i += 32 * 16) *reinterpret_cast<uint4*>(ring.tiles + i) = make_uint4(0, 0, 0, 0);
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");     // before the TMA unit writes there
   __syncwarp();
 }
@@ -269,7 +280,7 @@ __global__ void __launch_bounds__(kWarps * 32, D == 64 ? 6 : 3) fwd_kernel(const
   if (kOne) zero_tiles(ring);
   const Stride stride(p, gridDim.x * kWarps);
   Step s = first_step(p);
-  if (s.b < p.B) ring.issue(p, maps, s);
+  if (s.b < p.B) ring.issue(p, maps, nullptr, s);
   uint4 qa[J];
   float m = -INFINITY, lsum = 0.f;
   float acc[I][8][2];                               // [channel 8 (g + 8 i) + e][query 2 t + c]
@@ -285,7 +296,7 @@ __global__ void __launch_bounds__(kWarps * 32, D == 64 ? 6 : 3) fwd_kernel(const
       for (int j = 0; j < J; ++j) qa[j] = g < n_rows ? query_chunk<D>(ring.queries, g, t4 + 4 * j) : make_uint4(0, 0, 0, 0);
     }
     __syncwarp();                                   // the other stage and the query rows have been read
-    if (next.b < p.B) ring.issue(p, maps, next);
+    if (next.b < p.B) ring.issue(p, maps, nullptr, next);
     const unsigned char *kt = ring.stage(), *vt = kt + tile_bytes<D>();
     const int left = p.L - s.l0;                    // rows of the tile that exist (16 or more: all)
 
@@ -379,7 +390,7 @@ __global__ void __launch_bounds__(kWarps * 32, D == 64 ? 6 : 3) fwd_kernel(const
 // operand: 16 depth rows at once), so that P^T and dS^T are left operands of dV = P^T dO and
 // dK = dS^T Q as they come.
 template <typename T, int D, bool kOne, bool kAdd>
-__global__ void __launch_bounds__(kWarps * 32, D == 64 ? (kOne ? 5 : 4) : 3) bwd_kernel(const __grid_constant__ Params p, const __grid_constant__ Maps maps, const __grid_constant__ OutMaps omaps) {
+__global__ void __launch_bounds__(kWarps * 32, D == 64 ? (kAdd ? 3 : kOne ? 5 : 4) : 3) bwd_kernel(const __grid_constant__ Params p, const __grid_constant__ Maps maps, const __grid_constant__ OutMaps omaps) {
   constexpr int J = D / 32, I = D / 64;
   extern __shared__ __align__(1024) unsigned char smem[];
   if (smem_u32(smem) & 1023u) {
@@ -390,7 +401,8 @@ __global__ void __launch_bounds__(kWarps * 32, D == 64 ? (kOne ? 5 : 4) : 3) bwd
   const int lane = threadIdx.x & 31, g = lane >> 2, t4 = lane & 3;
   const int my_row = row_of(g >> 1, g & 1);         // tile row (+ 8) of this lane's operands and results
   const bool row_ok = g < p.G;
-  Ring<D, 3> ring(p, smem);
+  constexpr int NT = bwd_tiles<D, kAdd>();
+  Ring<D, 3, NT> ring(p, smem);
   if (kOne) zero_tiles(ring);
   const Stride stride(p, gridDim.x * kWarps);
   Step s = first_step(p);
@@ -400,7 +412,7 @@ __global__ void __launch_bounds__(kWarps * 32, D == 64 ? (kOne ? 5 : 4) : 3) bwd
   float dq[I][8][2];                                         // [channel 8 (g + 8 i) + e][query 2 t + c]
   bool ok = true;
   auto issue = [&](const Step& x) {
-    ring.issue(p, maps, x);
+    ring.issue(p, maps, &omaps, x);
     if (kOne || x.l0 == 0) {
       const float* l = p.lse + ((int64_t)x.b * p.T_q + x.t * p.G + 2 * t4) * p.H + x.h;
 #pragma unroll
@@ -501,8 +513,13 @@ __global__ void __launch_bounds__(kWarps * 32, D == 64 ? (kOne ? 5 : 4) : 3) bwd
       for (int nt = 0; nt < 2; ++nt)
         if (my_row + 8 * nt < left) {
           if (kAdd) {   // gradient cache shared by several layers: add to what earlier calls left
-            add8<T>(gk[nt], *reinterpret_cast<const uint4*>(dkb + 8 * nt * p.dkd.st + 32 * j));
-            add8<T>(gv[nt], *reinterpret_cast<const uint4*>(dvb + 8 * nt * p.dvd.st + 32 * j));
+            if constexpr (NT == 4) {
+              add8<T>(gk[nt], tile_chunk<kRows>(kt + 2 * tile_bytes<D>(), my_row + 8 * nt, t4 + 4 * j));
+              add8<T>(gv[nt], tile_chunk<kRows>(kt + 3 * tile_bytes<D>(), my_row + 8 * nt, t4 + 4 * j));
+            } else {
+              add8<T>(gk[nt], *reinterpret_cast<const uint4*>(dkb + 8 * nt * p.dkd.st + 32 * j));
+              add8<T>(gv[nt], *reinterpret_cast<const uint4*>(dvb + 8 * nt * p.dvd.st + 32 * j));
+            }
           }
           *reinterpret_cast<uint4*>(out + chunk_at<kRows>(my_row + 8 * nt, t4 + 4 * j)) = pack8<T>(gk[nt]);
           *reinterpret_cast<uint4*>(out + tile_bytes<D>() + chunk_at<kRows>(my_row + 8 * nt, t4 + 4 * j)) = pack8<T>(gv[nt]);

@@ -230,8 +230,9 @@ int fda_launch(K kernel, int id, size_t smem, int n_sm, cudaStream_t st, const P
 template <typename T, int D, bool kOne>
 int fda_run(const Params& p, const fda::Maps& maps, const fda::OutMaps& omaps, bool is_bwd, int n_sm, cudaStream_t st) {
   if (!is_bwd) return fda_launch(fda::fwd_kernel<T, D, kOne>, prof::kFdaFwd, fda::smem_bytes<D, 1>(p.G), n_sm, st, p, maps);
-  return fda_launch(p.acc_depth ? fda::bwd_kernel<T, D, kOne, true> : fda::bwd_kernel<T, D, kOne, false>, prof::kFdaBwd,
-                    fda::smem_bytes<D, 3>(p.G), n_sm, st, p, maps, omaps);
+  if (p.acc_depth)
+    return fda_launch(fda::bwd_kernel<T, D, kOne, true>, prof::kFdaBwd, fda::smem_bytes<D, 3, fda::bwd_tiles<D, true>()>(p.G), n_sm, st, p, maps, omaps);
+  return fda_launch(fda::bwd_kernel<T, D, kOne, false>, prof::kFdaBwd, fda::smem_bytes<D, 3>(p.G), n_sm, st, p, maps, omaps);
 }
 template <typename T>
 int fda_run_d(const Params& p, const fda::Maps& m, const fda::OutMaps& om, int D, bool is_bwd, int n_sm, cudaStream_t st) {
