@@ -71,6 +71,17 @@ __device__ __forceinline__ void bulk_commit() { asm volatile("cp.async.bulk.comm
 __device__ __forceinline__ void bulk_wait_read_all() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
 __device__ __forceinline__ void bulk_wait_all() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
 
+// The launches of a backward overlap at their ends (programmatic dependent launch): the next grid's CTAs
+// take the SMs that the last CTAs of this one leave idle.  pre -> dq -> dk/dv -> depth gradients: the
+// last three need what pre wrote and nothing of each other.
+//   grid_started  lets the next grid begin once every CTA of this one has got there (or has left)
+//   grid_before   waits for the grid before this one to be complete: dq calls it before it reads the
+//                 statistics and only then lets dk/dv begin, so that whoever begins later may read
+//                 them too; dk/dv and the depth gradients call it last, so that a grid never
+//                 ends before the ones that were launched ahead of it.
+__device__ __forceinline__ void grid_started() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void grid_before() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 // ------------------------------------------------------------------ statistics pass
 // delta = rowsum(o * dO) from the stored o, and lse, both transposed to [B, H, T_qp] so that the
 // backward kernels fetch 64 rows of one (b, h) with one 256-byte bulk copy.  Eight lanes per row,
@@ -79,6 +90,7 @@ __device__ __forceinline__ void bulk_wait_all() { asm volatile("cp.async.bulk.wa
 template <typename T, int D>
 __global__ void __launch_bounds__(256) pre_kernel(const __grid_constant__ Params p, float* delta_t, float* lse_t, float* norm_t, int T_qp) {
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, sub = lane & 7, grp = lane >> 3;
+  grid_started();
   const uint32_t groups_per_bh = (uint32_t)T_qp / 32u;             // T_qp is a multiple of 64
   const int64_t n_groups = (int64_t)p.B * p.H * groups_per_bh;
   for (int64_t gidx = blockIdx.x; gidx < n_groups; gidx += gridDim.x) {
@@ -198,6 +210,7 @@ dq_kernel(const __grid_constant__ Params p, const __grid_constant__ DqMaps maps,
   const uint32_t base = smem_u32(smem_raw);
   if (base & 1023u) {   // the 128-byte swizzle needs 1024-byte aligned tiles
     if (threadIdx.x == 0) record_failure(2 << 8);
+    grid_before();
     return;
   }
   const uint32_t sRing = base;
@@ -211,7 +224,7 @@ dq_kernel(const __grid_constant__ Params p, const __grid_constant__ DqMaps maps,
   volatile int* drain_flag = reinterpret_cast<volatile int*>(gctl + 8 * kMaxBars + 8);
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  if (launch_failed(p)) return;
+  if (launch_failed(p)) { grid_before(); return; }
 
   const int n_qt = (p.T_q + kBM - 1) / kBM;
   const BlockId bid = block_order(p, D);
@@ -262,6 +275,8 @@ dq_kernel(const __grid_constant__ Params p, const __grid_constant__ DqMaps maps,
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
+  grid_before();
+  grid_started();
   const uint32_t tmem = *tmem_slot;
   const uint32_t tmem_dQ = tmem + 256, tmem_Q = tmem + 384, tmem_dO = tmem + 448;
   constexpr uint32_t fmt = std::is_same<T, __nv_bfloat16>::value ? 1u : 0u;
@@ -547,6 +562,7 @@ dkv_kernel(const __grid_constant__ Params p, const __grid_constant__ DkvMaps map
   const uint32_t base = smem_u32(smem_raw);
   if (base & 1023u) {
     if (threadIdx.x == 0) record_failure(2 << 8);
+    grid_before();
     return;
   }
   const uint32_t sRing = base;
@@ -563,9 +579,10 @@ dkv_kernel(const __grid_constant__ Params p, const __grid_constant__ DkvMaps map
   volatile int* peer_failed = reinterpret_cast<volatile int*>(gctl + 8 * kMaxBars + 12);
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  if (!kSplit && launch_failed(p)) return;              // (a cluster stays together: below)
+  if (!kSplit && launch_failed(p)) { grid_before(); return; }   // (a cluster stays together: below)
   const int parts = kSplit ? (int)cluster_size() : 1, part = kSplit ? (int)cluster_rank() : 0;
 
+  grid_started();
   const BlockId bid = block_order(p, D, parts);
   const int h = bid.h, b = bid.b;
   const bool is_dep = bid.rank >= n_seq_key_tiles;
@@ -922,6 +939,7 @@ dkv_kernel(const __grid_constant__ Params p, const __grid_constant__ DkvMaps map
     tc_fence_after();
     tmem_dealloc(tmem, 512);
   }
+  if (tid == 0) grid_before();
 }
 
 // ==================================================================== depth dk / dv
@@ -990,6 +1008,7 @@ depth_grad_kernel(const __grid_constant__ Params p, const __grid_constant__ DkvM
   const uint32_t base = smem_u32(smem_raw);
   if (base & 1023u) {
     if (threadIdx.x == 0) record_failure(2 << 8);
+    grid_before();
     return;
   }
   const uint32_t sQ = base, sDO = base + kStepTile, sStat = base + 2 * kStepTile;
@@ -1003,7 +1022,7 @@ depth_grad_kernel(const __grid_constant__ Params p, const __grid_constant__ DkvM
   volatile int* drain_flag = reinterpret_cast<volatile int*>(gctl + 112);
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  if (launch_failed(p)) return;
+  if (launch_failed(p)) { grid_before(); return; }
 
   const int n_xb = (p.T_q + kStep - 1) / kStep;
   const int total = n_xb * p.H * p.B;                   // 64-row blocks; this CTA takes blockIdx.x, + gridDim.x, ...
@@ -1284,6 +1303,7 @@ depth_grad_kernel(const __grid_constant__ Params p, const __grid_constant__ DkvM
     tc_fence_after();
     tmem_dealloc(tmem, 512);
   }
+  if (tid == 0) grid_before();
 }
 
 // The query-stationary depth-gradient kernel owns its depth rows only when a 64-row block

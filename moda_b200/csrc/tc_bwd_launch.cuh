@@ -70,6 +70,33 @@ inline int dkv_parts(const Params& p, int n_sm) {
   return parts;
 }
 
+// `overlap`: the launch may begin when every CTA of the one before it has reached grid_started()
+// (tc_bwd_kernels.cuh says how the kernels keep their order); `parts` CTAs in x form a cluster.
+template <typename... KernelArgs, typename... Args>
+inline cudaError_t launch_next(void (*kern)(KernelArgs...), dim3 grid, int threads, size_t smem, int parts, bool overlap, cudaStream_t st,
+                               const Args&... args) {
+  cudaLaunchAttribute attr[2]{};
+  int n = 0;
+  if (overlap) {
+    attr[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[n++].val.programmaticStreamSerializationAllowed = 1;
+  }
+  if (parts > 1) {
+    attr[n].id = cudaLaunchAttributeClusterDimension;
+    attr[n].val.clusterDim.x = parts;
+    attr[n].val.clusterDim.y = attr[n].val.clusterDim.z = 1;
+    ++n;
+  }
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cfg.attrs = attr;
+  cfg.numAttrs = n;
+  return cudaLaunchKernelEx(&cfg, kern, args...);
+}
+
 template <typename T, int D>
 inline cudaError_t launch_bwd(const Params& p, const BwdMaps& m, const BwdBuffers& w, int T_qp, bool dg, bool fused,
                               int n_sm, cudaStream_t st, int* launches) {
@@ -78,6 +105,10 @@ inline cudaError_t launch_bwd(const Params& p, const BwdMaps& m, const BwdBuffer
   float* lse_t = w.lse_t;
   const int n_seq = (p.T_kv + kBN - 1) / kBN;
   const int n_dep_tiles = (int)(((int64_t)p.T_kv * p.L + kBN - 1) / kBN);
+  // The ends of a launch are a share of it that shrinks with the CTAs an SM works through: 12-layer stack of
+  // B = 2, T = 2048, H = 4, G = 4 (512 CTAs of dq) 3.79 -> 3.64 ms, B = 3, T = 1531, H = 5, G = 2 (360) 234 -> 220 us,
+  // T = 65536, G = 8, H = 8 (32768) 187.6 and 188.1 ms.
+  const bool overlap = !fused && (int64_t)((p.T_q + kBM - 1) / kBM) * p.H * p.B <= (int64_t)16 * n_sm;
   if (fused) {
     if constexpr (D == 128) {
       if ((e = cudaMemsetAsync(w.kvmax, 0, w.kvmax_bytes, st)) != cudaSuccess) return e;
@@ -145,28 +176,19 @@ inline cudaError_t launch_bwd(const Params& p, const BwdMaps& m, const BwdBuffer
       if ((e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dq_smem)) != cudaSuccess) return e;
       dim3 grid((p.T_q + kBM - 1) / kBM, p.H, p.B);
       prof::Scope ps(prof::kDqTc, st);
-      kern<<<grid, kDqThreads, dq_smem, st>>>(p, m.dq, delta_t, lse_t, T_qp, nullptr, nullptr);
+      e = launch_next(kern, grid, kDqThreads, dq_smem, 1, overlap, st, p, m.dq, (const float*)delta_t, (const float*)lse_t, T_qp, (const int*)nullptr,
+                      (const float4*)nullptr);
     }
-    if ((e = cudaGetLastError()) != cudaSuccess) return e;
+    if (e != cudaSuccess) return e;
     *launches += 1;
     {
       const bool own_tiles = !dg && n_dep_tiles > 0;
       const int parts = own_tiles ? 1 : dkv_parts(p, n_sm);
       auto kern = parts > 1 ? dkv_kernel<T, D, true> : dkv_kernel<T, D, false>;
       if ((e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dkv_smem)) != cudaSuccess) return e;
-      cudaLaunchConfig_t cfg{};
-      cfg.gridDim = dim3((n_seq + (own_tiles ? n_dep_tiles : 0)) * parts, p.H, p.B);
-      cfg.blockDim = dim3(kDkvThreads);
-      cfg.dynamicSmemBytes = dkv_smem;
-      cfg.stream = st;
-      cudaLaunchAttribute cluster{};
-      cluster.id = cudaLaunchAttributeClusterDimension;
-      cluster.val.clusterDim.x = parts;
-      cluster.val.clusterDim.y = cluster.val.clusterDim.z = 1;
-      cfg.attrs = &cluster;
-      cfg.numAttrs = parts > 1 ? 1 : 0;
+      const dim3 grid((n_seq + (own_tiles ? n_dep_tiles : 0)) * parts, p.H, p.B);
       prof::Scope ps(prof::kDkvTc, st);
-      e = cudaLaunchKernelEx(&cfg, kern, p, m.dkv, (const float*)delta_t, (const float*)lse_t, T_qp, n_seq);
+      e = launch_next(kern, grid, kDkvThreads, dkv_smem, parts, overlap, st, p, m.dkv, (const float*)delta_t, (const float*)lse_t, T_qp, n_seq);
     }
     if (e != cudaSuccess) return e;
     *launches += 1;
@@ -179,9 +201,9 @@ inline cudaError_t launch_bwd(const Params& p, const BwdMaps& m, const BwdBuffer
     dim3 grid((unsigned)(n_blocks < n_sm ? n_blocks : n_sm));
     {
       prof::Scope ps(prof::kDepthGradTc, st);
-      kern<<<grid, kDgThreads, smem, st>>>(p, m.dkv, m.out, delta_t, lse_t, T_qp);
+      e = launch_next(kern, grid, kDgThreads, smem, 1, overlap, st, p, m.dkv, m.out, (const float*)delta_t, (const float*)lse_t, T_qp);
     }
-    if ((e = cudaGetLastError()) != cudaSuccess) return e;
+    if (e != cudaSuccess) return e;
     *launches += 1;
   }
   return cudaSuccess;
