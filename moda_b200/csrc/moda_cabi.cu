@@ -257,14 +257,20 @@ int resolve_path(const moda_problem* pr, bool is_bwd) {
 
 int tc_forward(const Params& p, const moda_problem* prob, int n_sm, cudaStream_t st) {
   // Two forwards.  tc::fwd3 (two 128-row query tiles per CTA, one CTA per SM, one MMA warp
-  // ordering the work of both tiles) is the faster one once its grid fills the GPU; tc::fwd
-  // (one query tile per CTA, two CTAs per SM) has twice as many, smaller CTAs and serves the
-  // small problems.  Both use the same softmax arithmetic, so a result does not depend on the
+  // ordering the work of both tiles) is the faster one once its grid fills the GPU and a query tile
+  // has more than a few key tiles; tc::fwd (one query tile per CTA, two CTAs per SM) has twice as
+  // many, smaller CTAs and serves the small problems.  Both use the same softmax arithmetic, so a result does not depend on the
   // choice.  MODA_PATH_TCGEN05_ONE_TILE / _TWO_TILES force one of them.
   bool two_tiles = prob->path == MODA_PATH_TCGEN05_TWO_TILES;
   if (prob->path != MODA_PATH_TCGEN05_ONE_TILE && prob->path != MODA_PATH_TCGEN05_TWO_TILES) {
     const int64_t n_cta = (int64_t)((p.T_q + 255) / 256) * p.H * p.B;
-    two_tiles = n_sm > 0 && n_cta >= n_sm;
+    // mean key tiles of a 128-row query tile.  Up to 3 the kernels live on set-up, first loads and stores, and
+    // two CTAs an SM hide each other's.  One tile against two, us: 2 tiles (B = 256, T = 197, H = 6, all keys)
+    // D = 64: 102, 113, D = 128: 130, 139; 2.5 (B = 64, T = 512, H = 8, causal) 88, 102 and 107, 122; 3 (T = 384, all
+    // keys, D = 64) 63, 72; 4 (T = 512, all keys, D = 128) 116, 110; 8.5 (B = 2, T = 2048, H = 4, G = 4, D = 128) 59, 46.
+    const double seq_tiles = (p.T_kv + 127) / 128;
+    const double tiles = (p.mode == kNonCausal ? seq_tiles : 0.5 * (seq_tiles + 1)) + (double)p.L / p.G;
+    two_tiles = n_sm > 0 && n_cta >= n_sm && tiles > 3;
   }
   if (two_tiles) return tc::fwd3(p, prob, st, &g_last_launches, &g_last_cuda_error);
   return tc::fwd(p, prob, st, &g_last_launches, &g_last_cuda_error);
