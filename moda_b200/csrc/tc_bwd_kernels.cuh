@@ -426,7 +426,6 @@ dq_kernel(const __grid_constant__ Params p, const __grid_constant__ DqMaps maps,
       const bool is_dep = i >= n_seq;
       const int c0 = is_dep ? dep_c0 + (i - n_seq) * dep_rows : i * kStep;
       const bool masked = is_dep || (c0 + kStep > seq_full_hi);
-      const int lo = is_dep ? dlo : slo, hi = is_dep ? min(dhi, c0 + dep_rows) : shi;
       const uint32_t tS = tmem + (i & 1) * 128 + lane_addr;
       uint32_t su[64], du[64];
       tmem_ld32<0>(tS, su);
@@ -448,6 +447,7 @@ dq_kernel(const __grid_constant__ Params p, const __grid_constant__ DqMaps maps,
         pr[2 * jj + 1] = fast_exp2(x.y);
       }
       if (masked) {
+        const int lo = is_dep ? dlo : slo, hi = is_dep ? min(dhi, c0 + dep_rows) : shi;
 #pragma unroll
         for (int jj = 0; jj < 64; ++jj) {
           const int col = c0 + jj;

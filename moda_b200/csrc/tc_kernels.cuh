@@ -711,6 +711,11 @@ inline bool depth_layout_supported(const moda_problem* pr) {
   return pr->path == MODA_PATH_AUTO && pr->L <= 64;
 }
 inline bool fwd_supported(const moda_problem* pr) {
+  // One key tile of 64 rows at D = 64 and a layer count that needs boxes of whole positions: the 64-row tiles of
+  // the mma.sync forward do less padding (L = 5, G = 2, B = 64, H = 8: 35 us against 55; B = 1, H = 2, L = 3: 12.3
+  // against 14.4; at T = 128 14.4 against 13.8, at D = 128 T = 64 16.5 against 15.0).
+  if (pr->path == MODA_PATH_AUTO && pr->D == 64 && pr->T_kv <= 64 && pr->L > 0 && pr->depth_rows_per_pos > pr->L && 32 % pr->L != 0)
+    return false;
   return (pr->D == 128 || pr->D == 64) && pr->mode != MODA_DEPTH_ONLY && pr->scale > 0.f && depth_layout_supported(pr);
 }
 
