@@ -420,7 +420,8 @@ PyObject* py_cache_grads(PyObject*, PyObject* x) {
   END_HANDLE_TH_ERRORS
 }
 
-// cache_append(k, v, cache_k, cache_v, capacity, slot, token, state) -> token
+// cache_append(k, v, cache_k, cache_v, capacity, slot, token, state) -> token: the new one, or, where nothing is
+// recorded, the one that came in, which keeps the appends before it on the chain
 PyObject* py_cache_append(PyObject*, PyObject* const* a, Py_ssize_t n) {
   HANDLE_TH_ERRORS
   if (!arg_count(n, 8)) return nullptr;
@@ -432,7 +433,7 @@ PyObject* py_cache_append(PyObject*, PyObject* const* a, Py_ssize_t n) {
   op.scale = 1.;
   const int slot = as_int(a[5]);
   const CacheStatePtr state = as_state(a[7]);
-  Tensor next;
+  Tensor next = token;
   {
     NoGil no_gil;
     refuse_tangents({&k, &v});
@@ -446,7 +447,7 @@ PyObject* py_cache_append(PyObject*, PyObject* const* a, Py_ssize_t n) {
       check_status(moda_b200_depth_append(&pr, T4(k_).p(), T4(v_).p(), T4(cache_k).p(), T4(cache_v).p(), slot,
                                           c10::cuda::getCurrentCUDAStream().stream()),
                    "moda_b200_depth_append");
-      next = at::empty({}, k.options().dtype(at::kFloat));       // only its place in the graph is used
+      if (grad) next = at::empty({}, k.options().dtype(at::kFloat));       // only its place in the graph is used
     }
     if (grad) {
       std::shared_ptr<MoDADepthAppendBackward> node(new MoDADepthAppendBackward(), torch::autograd::deleteNode);
