@@ -19,6 +19,7 @@
 
 #include <ATen/core/Tensor.h>
 #include <ATen/ops/empty.h>
+#include <c10/core/Event.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/Exceptions.h>
@@ -31,6 +32,7 @@
 #include <atomic>
 #include <cmath>
 #include <memory>
+#include <optional>
 
 #include "../../include/moda_b200.h"
 
@@ -153,9 +155,22 @@ Grads run_backward(const Op& op, const Tensor& q_, const Tensor& k_, const Tenso
 // layers hold gradients: the first attention whose backward runs (as a rule the last layer, which
 // read every slot) stores its depth gradients there, the others add theirs, so that nothing has
 // to be zeroed; a later one that read more layers than are filled gets those zeroed first.
+// They pass from node to node outside the engine's sight, which orders two nodes' streams only along
+// defined gradients: whoever uses them on another stream than the last user waits for that one.
 struct CacheState {
   Tensor grad_k, grad_v;
   int filled = 0;
+  std::optional<c10::cuda::CUDAStream> last;       // stream of the last use
+  void used_on(const c10::cuda::CUDAStream& now) {
+    if (last && *last != now) {
+      c10::Event event(c10::DeviceType::CUDA);
+      event.record(last->unwrap());
+      event.block(now.unwrap());
+      grad_k.record_stream(now.unwrap());
+      grad_v.record_stream(now.unwrap());
+    }
+    last = now;
+  }
 };
 using CacheStatePtr = std::shared_ptr<CacheState>;
 
@@ -188,6 +203,7 @@ struct MoDAAttentionBackward : public Node {
         state->grad_k = at::empty(cache_k.sizes(), cache_k.options());
         state->grad_v = at::empty(cache_v.sizes(), cache_v.options());
       }
+      state->used_on(c10::cuda::getCurrentCUDAStream(q_.device().index()));
       if (state->filled == 0) {
         accumulate = false;
       } else if (op.layers > state->filled) {
@@ -224,6 +240,7 @@ struct MoDADepthAppendBackward : public Node {
     if (!state->grad_k.defined() || slot >= state->filled) return out;      // no attention that read the slot has run
     at::AutoGradMode no_grad(false);
     const Tensor& gk = state->grad_k;
+    state->used_on(c10::cuda::getCurrentCUDAStream(gk.device().index()));
     const std::vector<int64_t> shape{gk.size(0), pr.T_kv, gk.size(2), gk.size(3)};
     out[0] = at::empty(shape, gk.options());
     out[1] = at::empty(shape, gk.options());

@@ -29,17 +29,20 @@ def _rebuilt(layers, frozen=()):
     return outs
 
 
-def _cached(layers, frozen=()):
-    """The same through the in-place cache."""
+def _cached(layers, frozen=(), streams=lambda i: (None, None)):
+    """The same through the in-place cache, layer i's attention and append on `streams(i)`."""
     import moda_b200 as M
     cache = M.DepthKVCache(2, T, len(layers) - 1, H, D, torch.bfloat16, "cuda")
     outs = []
     for i, (q, k, v) in enumerate(layers):
-        with torch.set_grad_enabled(i not in frozen):
+        attend_on, append_on = streams(i)
+        with torch.cuda.stream(attend_on), torch.set_grad_enabled(i not in frozen):
             outs.append(cache.attend(q, k, v, moda_group_num=G))
         if i + 1 < len(layers):
-            with torch.set_grad_enabled(i not in frozen):
+            with torch.cuda.stream(append_on), torch.set_grad_enabled(i not in frozen):
                 cache.append(k, v)
+        if attend_on is not None:
+            torch.cuda.synchronize()             # the forward's own order is the caller's to keep
     return outs
 
 
@@ -57,3 +60,25 @@ def test_layers_that_are_not_recorded(built_library, frozen):
     got, want = [torch.autograd.grad([outs[i] for i in live], leaves, [dout[i] for i in live])
                  for outs in (_cached(layers, frozen), _rebuilt(layers, frozen))]
     _check(got, want)
+
+
+@pytest.mark.parametrize("which", ["append", "layers"])
+def test_streams(built_library, which):
+    """The gradient cache is ordered between the streams that the backward runs on: here every attention's
+    share of it comes late."""
+    layers, dout = _leaves(2, 5)
+    leaves = [x for lay in layers for x in lay]
+    main, side = torch.cuda.Stream(), torch.cuda.Stream()
+    torch.cuda.synchronize()
+    streams = (lambda i: (main, side)) if which == "append" else (lambda i: (main, side) if i % 2 else (side, side))
+    outs = _cached(layers, streams=streams)
+
+    def late(grad):
+        torch.cuda._sleep(4_000_000)
+        return grad
+
+    for o in outs:
+        o.register_hook(late)
+    got = torch.autograd.grad(outs, leaves, dout)
+    torch.cuda.synchronize()
+    _check(got, torch.autograd.grad(_rebuilt(layers), leaves, dout))
