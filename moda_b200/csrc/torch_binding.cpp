@@ -26,6 +26,7 @@
 #include <torch/csrc/autograd/function.h>
 #include <torch/csrc/autograd/functions/utils.h>
 #include <torch/csrc/autograd/grad_mode.h>
+#include <torch/csrc/autograd/graph_task.h>
 #include <torch/csrc/autograd/python_variable.h>
 #include <torch/csrc/autograd/saved_variable.h>
 
@@ -155,12 +156,19 @@ Grads run_backward(const Op& op, const Tensor& q_, const Tensor& k_, const Tenso
 // layers hold gradients: the first attention whose backward runs (as a rule the last layer, which
 // read every slot) stores its depth gradients there, the others add theirs, so that nothing has
 // to be zeroed; a later one that read more layers than are filled gets those zeroed first.
+// They belong to one run of the engine: a second one over the same forward (a retained graph, losses of
+// single layers) starts with caches of its own, and hands on nothing that an earlier one left.
 // They pass from node to node outside the engine's sight, which orders two nodes' streams only along
 // defined gradients: whoever uses them on another stream than the last user waits for that one.
 struct CacheState {
   Tensor grad_k, grad_v;
   int filled = 0;
+  int run = -1;                                    // the engine's number of its run
   std::optional<c10::cuda::CUDAStream> last;       // stream of the last use
+  void enter(int now) {
+    if (run != now) *this = CacheState();
+    run = now;
+  }
   void used_on(const c10::cuda::CUDAStream& now) {
     if (last && *last != now) {
       c10::Event event(c10::DeviceType::CUDA);
@@ -199,6 +207,7 @@ struct MoDAAttentionBackward : public Node {
     Grads g;
     if (state && op.layers > 0) {
       bool accumulate = true;
+      state->enter(torch::autograd::get_current_graph_task_id());
       if (!state->grad_k.defined()) {
         state->grad_k = at::empty(cache_k.sizes(), cache_k.options());
         state->grad_v = at::empty(cache_v.sizes(), cache_v.options());
@@ -237,6 +246,7 @@ struct MoDADepthAppendBackward : public Node {
   std::string name() const override { return "MoDADepthAppendBackward"; }
   variable_list apply(variable_list&&) override {
     variable_list out(3);
+    state->enter(torch::autograd::get_current_graph_task_id());
     if (!state->grad_k.defined() || slot >= state->filled) return out;      // no attention that read the slot has run
     at::AutoGradMode no_grad(false);
     const Tensor& gk = state->grad_k;

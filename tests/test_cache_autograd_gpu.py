@@ -82,3 +82,25 @@ def test_streams(built_library, which):
     got = torch.autograd.grad(outs, leaves, dout)
     torch.cuda.synchronize()
     _check(got, torch.autograd.grad(_rebuilt(layers), leaves, dout))
+
+
+@pytest.mark.parametrize("how", ["twice", "one leaf first", "a loss a layer"])
+def test_several_backwards_of_one_forward(built_library, how):
+    """Each delivers its own gradients once."""
+    layers, dout = _leaves(3, 4)
+    leaves = [x for lay in layers for x in lay]
+
+    def backwards(outs):
+        if how == "twice":
+            torch.autograd.grad(outs, leaves, dout, retain_graph=True)
+        elif how == "one leaf first":
+            torch.autograd.grad(outs[-1], layers[-1][0], dout[-1], retain_graph=True)
+        else:
+            for x in leaves:
+                x.grad = None
+            for o, d in zip(outs, dout):
+                o.backward(d)
+            return [x.grad for x in leaves]
+        return torch.autograd.grad(outs, leaves, dout)
+
+    _check(backwards(_cached(layers)), backwards(_rebuilt(layers)))
