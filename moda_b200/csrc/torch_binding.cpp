@@ -362,14 +362,19 @@ bool well_formed(const Tensor& q, const Tensor& k, const Tensor& v, Tensor& ck, 
 }
 
 // attention(q, k, v, cached_k, cached_v, scale, G, mode, return_depth_grads, warn_shape, checked)
-//   -> (o, lse), or None for a call that the Python wrapper has to look at (never when `checked`)
+//   -> (o, lse), or None for a call that the Python wrapper has to look at (never when `checked`).
+// G is anything with __index__ (a NumPy integer, say).
 PyObject* py_attention(PyObject*, PyObject* const* a, Py_ssize_t n) {
   HANDLE_TH_ERRORS
   if (!arg_count(n, 11)) return nullptr;
   const bool checked = a[10] == Py_True;
   for (int i = 0; i < 5; ++i)
-    if (!tensor_or_none_check(a[i])) Py_RETURN_NONE;
-  if (!PyLong_Check(a[6]) || !(a[5] == Py_None || PyFloat_Check(a[5]) || PyLong_Check(a[5]))) Py_RETURN_NONE;
+    if (!tensor_or_none_check(a[i])) {
+      if (!checked) Py_RETURN_NONE;
+      PyErr_SetString(PyExc_TypeError, "moda_b200: the operands must be tensors");
+      return nullptr;
+    }
+  if (!checked && !(PyIndex_Check(a[6]) && (a[5] == Py_None || PyFloat_Check(a[5]) || PyLong_Check(a[5])))) Py_RETURN_NONE;
   const Tensor q = tensor_or_none(a[0]), k = tensor_or_none(a[1]), v = tensor_or_none(a[2]);
   Tensor ck = tensor_or_none(a[3]), cv = tensor_or_none(a[4]);
   Op op;
