@@ -13,7 +13,7 @@
 //   attention(q, k, v, cached_k, cached_v, scale, G, mode, return_depth_grads, warn_shape, checked)
 //   forward(q, k, v, cached_k, cached_v, scale, G, mode, chunk_rows)
 //   backward(q, k, v, cached_k, cached_v, o, lse, dout, scale, G, mode, chunk_rows)
-//   cache_state(), cache_grads(state), cache_append(...), cache_attention(...): DepthKVCache
+//   cache_state([grad_k, grad_v]), cache_grads(state), cache_append(...), cache_attention(...): DepthKVCache
 //   set_path(path), set_check(fn)
 #include <Python.h>
 
@@ -439,9 +439,16 @@ CacheStatePtr as_state(PyObject* x) {
   if (!p) throw python_error();
   return *p;
 }
-PyObject* py_cache_state(PyObject*, PyObject*) {
+// cache_state() -> a new state; cache_state(grad_k, grad_v): with these gradient caches (a copy of another's)
+PyObject* py_cache_state(PyObject*, PyObject* const* a, Py_ssize_t n) {
   HANDLE_TH_ERRORS
-  return PyCapsule_New(new CacheStatePtr(std::make_shared<CacheState>()), kStateName,
+  if (n != 0 && !arg_count(n, 2)) return nullptr;
+  auto state = std::make_shared<CacheState>();
+  if (n != 0) {
+    state->grad_k = tensor_or_none(a[0]);
+    state->grad_v = tensor_or_none(a[1]);
+  }
+  return PyCapsule_New(new CacheStatePtr(std::move(state)), kStateName,
                        [](PyObject* c) { delete static_cast<CacheStatePtr*>(PyCapsule_GetPointer(c, kStateName)); });
   END_HANDLE_TH_ERRORS
 }
@@ -530,7 +537,7 @@ PyObject* py_set_check(PyObject*, PyObject* x) {
 PyMethodDef kMethods[] = {{"attention", MODA_FAST(py_attention), nullptr},
                           {"forward", MODA_FAST(py_forward), nullptr},
                           {"backward", MODA_FAST(py_backward), nullptr},
-                          {"cache_state", py_cache_state, METH_NOARGS, nullptr},
+                          {"cache_state", MODA_FAST(py_cache_state), nullptr},
                           {"cache_grads", py_cache_grads, METH_O, nullptr},
                           {"cache_append", MODA_FAST(py_cache_append), nullptr},
                           {"cache_attention", MODA_FAST(py_cache_attention), nullptr},

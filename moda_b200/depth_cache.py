@@ -69,6 +69,18 @@ class DepthKVCache:
             self._state = _cabi.native().cache_state()
         return self._state
 
+    # Copies and pickles hold the gradient caches as tensors: the native state is one of this process.
+    def __getstate__(self):
+        state = dict(self.__dict__)
+        if self._state is not None:
+            state["_state"] = tuple(_cabi.native().cache_grads(self._state))
+        return state
+
+    def __setstate__(self, state):
+        self.__dict__.update(state)
+        if state["_state"] is not None:
+            self._state = _cabi.native().cache_state(*state["_state"])
+
     def bytes_copied_per_forward(self, n_layers: int) -> int:
         """Bytes of K/V this cache copies for a model of ``n_layers`` attention layers (each of the
         first n_layers - 1 layers once)."""

@@ -1,6 +1,9 @@
 """GPU: gradients of a stack of layers over ``DepthKVCache`` when the pass is not the plain one (every layer
 recorded, on one stream, one backward).  Reference: the packed cache rebuilt before every layer
 (``torch.stack`` of the earlier layers' K/V) through the ordinary operator."""
+import copy
+import pickle
+
 import pytest
 import torch
 
@@ -104,3 +107,30 @@ def test_several_backwards_of_one_forward(built_library, how):
         return torch.autograd.grad(outs, leaves, dout)
 
     _check(backwards(_cached(layers)), backwards(_rebuilt(layers)))
+
+
+@pytest.mark.parametrize("how", ["deepcopy", "pickle"])
+@pytest.mark.parametrize("train", [False, True])
+def test_copies_of_a_used_cache(built_library, how, train):
+    """A module that keeps one stays copyable; what was recorded stays with the original."""
+    import moda_b200 as M
+    layers, dout = _leaves(4, 3)
+    cache = M.DepthKVCache(2, T, 3, H, D, torch.bfloat16, "cuda")
+    with torch.set_grad_enabled(train):
+        for q, k, v in layers[:2]:
+            o = cache.attend(q, k, v, moda_group_num=G)
+            cache.append(k, v)
+    if train:
+        o.backward(dout[0])
+        if how == "deepcopy":                    # a tensor with a history, as ever
+            with pytest.raises(RuntimeError):
+                copy.deepcopy(cache)
+            return
+    other = copy.deepcopy(cache) if how == "deepcopy" else pickle.loads(pickle.dumps(cache))
+    assert other.L == 2 and other.k.data_ptr() != cache.k.data_ptr()
+    assert (other.grad_k is None) == (not train)
+    if train:                                    # the first backward filled one layer of three
+        at = lambda x: x.view(2, T, 3, H, D)[:, :, 0]  # noqa: E731
+        assert torch.equal(at(other.grad_k), at(cache.grad_k)) and torch.equal(at(other.grad_v), at(cache.grad_v))
+    with torch.no_grad():
+        assert torch.equal(other.attend(*layers[2], moda_group_num=G), cache.attend(*layers[2], moda_group_num=G))
