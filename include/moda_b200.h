@@ -216,7 +216,8 @@ int moda_b200_depth_take(const moda_problem *prob, const moda_tensor4 *grad_k,
 int moda_b200_check_problem(const moda_problem *prob);
 
 /* Which kernel path MODA_PATH_AUTO resolves to for this problem's forward (is_bwd=0)
- * or backward (is_bwd=1): MODA_PATH_SIMT_MMA or MODA_PATH_TCGEN05; <0 on bad input. */
+ * or backward (is_bwd=1): MODA_PATH_SIMT_MMA or MODA_PATH_TCGEN05; <0 on bad input.  Where the
+ * bandwidth kernels take the depth rows, the path of the sequence part. */
 int moda_b200_resolve_path(const moda_problem *prob, int is_bwd);
 
 /*

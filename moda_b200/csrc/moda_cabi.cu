@@ -358,7 +358,8 @@ int moda_b200_check_problem(const moda_problem* prob) { return check_problem(pro
 
 int moda_b200_resolve_path(const moda_problem* prob, int is_bwd) {
   if (int rc = check_problem(prob)) return -rc;
-  return resolve_path(prob, is_bwd != 0);
+  const moda_problem att = attention_problem(prob, is_bwd != 0);       // what the calls resolve on
+  return resolve_path(&att, is_bwd != 0);
 }
 
 int moda_b200_fwd(const moda_problem* prob, const moda_tensor4* q, const moda_tensor4* k,

@@ -183,6 +183,18 @@ def test_depth_cache_layout_fields_are_validated(lib):
     assert lib.moda_b200_depth_append(r(_prob(depth_rows_per_pos=11)), None, r(t4), r(t4), r(t4), 0, None) == 1
 
 
+@pytest.mark.parametrize("kw,bwd,path", [
+    (dict(L=3, depth_rows_per_pos=11), 0, 2),                # G = 1: the depth rows are split off, whatever their layout
+    (dict(L=3, depth_rows_per_pos=11), 1, 2),
+    (dict(L=70, depth_rows_per_pos=80, D=128), 1, 2),
+    (dict(L=70, depth_rows_per_pos=80, D=128, G=2), 1, 1),   # more layers than a step tile has rows
+    (dict(L=3, depth_rows_per_pos=11, G=2, T_kv=65), 0, 2),
+    (dict(L=3, depth_rows_per_pos=11, mode=2), 0, 1),        # chunk-visible depth is not split off
+])
+def test_resolve_path_is_what_the_calls_take(lib, kw, bwd, path):
+    assert lib.moda_b200_resolve_path(ctypes.byref(_prob(**kw)), bwd) == path
+
+
 def test_product_package_does_not_import_the_oracle():
     pkg = os.path.join(ROOT, "moda_b200")
     for dirpath, _, files in os.walk(pkg):
