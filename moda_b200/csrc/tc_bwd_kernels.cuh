@@ -619,7 +619,7 @@ dkv_kernel(const __grid_constant__ Params p, const __grid_constant__ DkvMaps map
       mbar_init(bars + 8 * (B_.p0 + i), 128);
       mbar_init(bars + 8 * (B_.r0 + i), 128); mbar_init(bars + 8 * (B_.t0 + i), 1);
     }
-    *abort_flag = kSplit && launch_failed(p) ? 1 : 0;
+    *abort_flag = kSplit && failure_published(p) ? 1 : 0;
     *drain_flag = 0;
     if (kSplit) *peer_failed = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");

@@ -61,8 +61,14 @@ __device__ __forceinline__ void record_failure(int code) {
   atomicCAS(&g_tc_sticky, 0, code);
 }
 
-__device__ __forceinline__ bool launch_failed(const Params& p) {
+__device__ __forceinline__ bool failure_published(const Params& p) {
   return *reinterpret_cast<volatile int*>(&g_tc_failed) == p.launch_id;
+}
+// One answer for the whole CTA, from all of its threads: the word may change between two threads' loads, and
+// a warp that leaves in part, or a CTA without some of its warps, breaks the collectives and
+// arrival counts of those that stay.
+__device__ __forceinline__ bool launch_failed(const Params& p) {
+  return __syncthreads_or(threadIdx.x == 0 && failure_published(p)) != 0;
 }
 __device__ __forceinline__ void publish_failure(const Params& p, volatile int* abort_flag) {
   if (*abort_flag != 0) atomicExch(&g_tc_failed, p.launch_id);

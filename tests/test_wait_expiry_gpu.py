@@ -71,11 +71,66 @@ def test_expired_wait_is_reported_and_context_survives(built_library, fwd):
     assert _cabi.device_status() == 0
 
 
+def _wait_test_library():
+    from moda_b200 import _cabi, build
+    wt = ctypes.CDLL(build.build_wait_test())
+    P, T4, V = ctypes.POINTER(_cabi.Problem), ctypes.POINTER(_cabi.Tensor4), ctypes.c_void_p
+    wt.moda_b200_fwd.argtypes = [P, T4, T4, T4, T4, T4, T4, V, V]
+    wt.moda_b200_bwd_workspace_bytes.argtypes = [P, ctypes.POINTER(ctypes.c_size_t)]
+    wt.moda_b200_bwd.argtypes = [P] + [T4] * 6 + [V] + [T4] * 6 + [V, ctypes.c_size_t, V]
+    wt.moda_b200_device_status.argtypes = [ctypes.POINTER(ctypes.c_int)]
+    return wt
+
+
+def _status(wt):
+    st = ctypes.c_int(-1)
+    assert wt.moda_b200_device_status(ctypes.byref(st)) == 0
+    return st.value
+
+
+def _t4(x):
+    from moda_b200 import _cabi
+    return ctypes.byref(_cabi.Tensor4(x.data_ptr(), x.stride(0), x.stride(1), x.stride(2)))
+
+
+def _elapsed_ms(call):
+    a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+    a.record()
+    call()
+    b.record()
+    torch.cuda.synchronize()
+    return a.elapsed_time(b)
+
+
+@pytest.mark.parametrize("fwd", ["one_tile", "two_tiles"])
+def test_blocks_that_start_after_a_failure_leave_at_once(built_library, fwd):
+    """Many more CTAs than the GPU holds: the first ones wait for the limit, the others see the call's number
+    and return, all threads of a CTA alike."""
+    from moda_b200 import _cabi
+    wt = _wait_test_library()
+    T, D = 64, 128
+    path = _cabi.PATH_TCGEN05_ONE_TILE if fwd == "one_tile" else _cabi.PATH_TCGEN05_TWO_TILES
+    ms = {}
+    for B, H in ((1, 1), (1, 1), (128, 32)):        # the first call loads the kernel
+        q, k, v = [torch.randn(B, T, H, D, device="cuda", dtype=torch.bfloat16) for _ in range(3)]
+        o, lse = torch.zeros_like(q), torch.zeros(B, T, H, dtype=torch.float32, device="cuda")
+        prob = _cabi.Problem(B, T, H, D, 1, 0, _cabi.MODE_CAUSAL, 64, _cabi.DTYPE_BF16, path, D ** -0.5, 0)
+
+        def call():
+            assert wt.moda_b200_fwd(ctypes.byref(prob), _t4(q), _t4(k), _t4(v), None, None, _t4(o), lse.data_ptr(),
+                                    torch.cuda.current_stream().cuda_stream) == 0
+
+        ms[B] = _elapsed_ms(call)
+        assert _status(wt) >> 8 == 1 and _status(wt) == 0
+        assert float(o.abs().max()) == 0.0
+    assert ms[128] < 4 * ms[1], ms               # 14 rounds of CTAs (one tile), 28 (two tiles)
+
+
 def test_expired_wait_in_the_backward_is_reported_and_context_survives(built_library):
     """The same for the backward: the test build's dq kernel withholds the softmax warps' "dS tile
     ready" arrival, the update-MMA warp's bounded wait runs out after about a millisecond, the CTA
-    frees its TMEM and returns, the dk/dv launch behind it sees the status word and returns at
-    once; no gradient is written, the status names the barrier, and the ordinary library then runs
+    frees its TMEM and returns; the dk/dv launch behind it, whose CTAs see that the call has failed or,
+    if they began before it did, wait for their own withheld arrival, returns too; no gradient is written, the status names the barrier, and the ordinary library then runs
     the same backward correctly."""
     import moda_b200 as M
     from moda_b200 import _cabi, build
