@@ -102,6 +102,42 @@ def _elapsed_ms(call):
     return a.elapsed_time(b)
 
 
+def _failing_backward(wt, B, T, H, D):
+    """A call of the wait-expiry build's backward and the gradients it must leave alone."""
+    import moda_b200 as M
+    from moda_b200 import _cabi
+    q, k, v, dout = [torch.randn(B, T, H, D, device="cuda", dtype=torch.bfloat16) for _ in range(4)]
+    o, lse = M.parallel_moda_fwd(q, k, v)
+    prob = _cabi.Problem(B, T, H, D, 1, 0, _cabi.MODE_CAUSAL, 64, _cabi.DTYPE_BF16, _cabi.PATH_TCGEN05, D ** -0.5, 0)
+    need = ctypes.c_size_t(0)
+    assert wt.moda_b200_bwd_workspace_bytes(ctypes.byref(prob), ctypes.byref(need)) == 0
+    ws = torch.empty(need.value, dtype=torch.uint8, device="cuda")
+    grads = [torch.zeros_like(x) for x in (q, k, v)]
+
+    def call():
+        assert wt.moda_b200_bwd(ctypes.byref(prob), _t4(q), _t4(k), _t4(v), None, None, _t4(o), lse.data_ptr(), _t4(dout),
+                                *[_t4(g) for g in grads], None, None, ws.data_ptr(), ws.numel(),
+                                torch.cuda.current_stream().cuda_stream) == 0
+
+    return call, grads
+
+
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("B,T,H", [(1, 512, 1),        # dk/dv: four tiles of two CTAs each
+                                   (1, 1024, 2),       # of four
+                                   (8, 128, 32)])      # more CTAs than SMs, no clusters
+def test_failed_backward_with_clusters(built_library, B, T, H, D):
+    """CTAs that share a key tile leave together when their waits run out, and store nothing."""
+    from moda_b200 import _cabi
+    wt = _wait_test_library()
+    call, grads = _failing_backward(wt, B, T, H, D)
+    call()
+    torch.cuda.synchronize()
+    assert _status(wt) >> 8 == 1 and _status(wt) == 0
+    assert all(float(g.abs().max()) == 0.0 for g in grads)
+    assert _cabi.device_status() == 0
+
+
 @pytest.mark.parametrize("fwd", ["one_tile", "two_tiles"])
 def test_blocks_that_start_after_a_failure_leave_at_once(built_library, fwd):
     """Many more CTAs than the GPU holds: the first ones wait for the limit, the others see the call's number
