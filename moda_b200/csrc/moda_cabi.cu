@@ -317,6 +317,18 @@ struct DeviceGuard {
   ~DeviceGuard() { int cur = -1; if (cudaGetDevice(&cur) == cudaSuccess && cur != prev && prev >= 0) cudaSetDevice(prev); }
 };
 
+// A captured call keeps its number from replay to replay, so that what a failed replay has published would end
+// every later one before it began: a node of the graph clears the word first.
+int clear_failure_if_captured(cudaStream_t st) {
+  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(st, &capture) != cudaSuccess) { cudaGetLastError(); return MODA_OK; }   // the launch will say
+  if (capture != cudaStreamCaptureStatusActive) return MODA_OK;
+  void* word = nullptr;
+  MODA_CUDA(cudaGetSymbolAddress(&word, tc::g_tc_failed));
+  MODA_CUDA(cudaMemsetAsync(word, 0, sizeof(int), st));
+  return MODA_OK;
+}
+
 // One layer's rows into (kTake: out of) slot `layer` of the caches.
 template <bool kTake>
 int cache_slot(const moda_problem* prob, const moda_tensor4* k, const moda_tensor4* v, const moda_tensor4* cache_k,
@@ -393,6 +405,7 @@ int moda_b200_fwd(const moda_problem* prob, const moda_tensor4* q, const moda_te
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   const int n_sm = sm_count(prob->device);
   if (n_sm <= 0) return cuda_fail(cudaErrorInvalidDevice);
+  if (int rc = clear_failure_if_captured(st)) return rc;
   if (use_fda(prob, false))
     return fda_dispatch(p, prob, false, n_sm, st);
   if (split_depth(prob, false)) {
@@ -463,6 +476,7 @@ int moda_b200_bwd(const moda_problem* prob, const moda_tensor4* q, const moda_te
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   const int n_sm = sm_count(prob->device);
   if (n_sm <= 0) return cuda_fail(cudaErrorInvalidDevice);
+  if (int rc = clear_failure_if_captured(st)) return rc;
   if (use_fda(prob, true))
     return fda_dispatch(p, prob, true, n_sm, st);
   if (split_depth(prob, true)) {   // depth rows' dq share, d_depth_k, d_depth_v; then the sequence part

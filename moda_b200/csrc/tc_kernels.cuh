@@ -51,7 +51,8 @@ template <int D> __host__ __device__ constexpr uint32_t tile_bytes() { return (u
 
 // g_tc_failed is the number (Params::launch_id) of the call in which a wait expired last, written by the
 // CTA's teardown: CTAs of that call's launches which start later return at once, and other calls,
-// whose numbers differ, need nothing cleared before they are enqueued.  g_tc_sticky keeps the first
+// whose numbers differ, need nothing cleared before they are enqueued (a captured call, whose number stays,
+// clears the word in its graph).  g_tc_sticky keeps the first
 // failure of any launch, (code << 8) | barrier id of the wait that expired, until the host reads it
 // (moda_b200_device_status), so that a later call cannot erase it.
 __device__ int g_tc_failed;
@@ -771,7 +772,7 @@ inline int read_status(int* out) {
   if (v != 0) {
     const int zero = 0;
     e = cudaMemcpyToSymbol(g_tc_sticky, &zero, sizeof(int));
-    if (e == cudaSuccess) e = cudaMemcpyToSymbol(g_tc_failed, &zero, sizeof(int));   // a captured call may be replayed
+    if (e == cudaSuccess) e = cudaMemcpyToSymbol(g_tc_failed, &zero, sizeof(int));
     if (e != cudaSuccess) return (int)e;
   }
   *out = v;

@@ -219,3 +219,31 @@ def test_expired_wait_in_the_backward_is_reported_and_context_survives(built_lib
         if a is not None:
             assert torch.equal(a, b)
     assert _cabi.device_status() == 0
+
+
+@pytest.mark.parametrize("bwd", [False, True])
+def test_a_captured_call_runs_again_after_a_failure(built_library, bwd):
+    """The call's number is part of the graph: what a replay left there does not stop the next one, which here
+    waits for the limit again."""
+    from moda_b200 import _cabi
+    wt = _wait_test_library()
+    B, T, H, D = 1, 64, 1, 128
+    if bwd:
+        call, _ = _failing_backward(wt, B, T, H, D)
+    else:
+        q, k, v = [torch.randn(B, T, H, D, device="cuda", dtype=torch.bfloat16) for _ in range(3)]
+        o, lse = torch.zeros_like(q), torch.zeros(B, T, H, dtype=torch.float32, device="cuda")
+        prob = _cabi.Problem(B, T, H, D, 1, 0, _cabi.MODE_CAUSAL, 64, _cabi.DTYPE_BF16, _cabi.PATH_TCGEN05, D ** -0.5, 0)
+
+        def call():
+            assert wt.moda_b200_fwd(ctypes.byref(prob), _t4(q), _t4(k), _t4(v), None, None, _t4(o), lse.data_ptr(),
+                                    torch.cuda.current_stream().cuda_stream) == 0
+    call()                                           # the first call loads the kernels
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        call()
+    _elapsed_ms(graph.replay)
+    first, second = _elapsed_ms(graph.replay), _elapsed_ms(graph.replay)
+    assert min(first, second) > 0.1, (first, second)  # a wait's limit; a launch that leaves at once takes 0.01
+    assert _status(wt) >> 8 == 1 and _status(wt) == 0
