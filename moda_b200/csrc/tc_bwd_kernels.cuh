@@ -267,7 +267,7 @@ dq_kernel(const __grid_constant__ Params p, const __grid_constant__ DqMaps maps,
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   }
-  if (n_dep > 0 && dep_rows < kStep) zero_tails(smem_raw, R * 2 * (D / 64), kStep, dep_rows);
+  if (n_dep > 0 && dep_rows < kStep) zero_tails(smem_raw, R * 2 * (D / 64), kStep, dep_rows, tid, blockDim.x);
   if (warp == 0) {
     tmem_alloc(bars + 8 * kMaxBars, 512);
     tmem_relinquish();

@@ -171,7 +171,6 @@ fwd3_kernel(const __grid_constant__ Params p, const __grid_constant__ Fwd3Maps m
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   }
-  if (pl.n > pl.n_s && pl.dep_rows < kBN) zero_tails(smem_raw + (2 + KS) * kTile, 2 * (D / 64), kBN, pl.dep_rows);   // V
   if (warp == 0) {
     tmem_alloc(bars + 8 * kMaxBars, 512);
     tmem_relinquish();
@@ -209,6 +208,11 @@ fwd3_kernel(const __grid_constant__ Params p, const __grid_constant__ Fwd3Maps m
         f3_step(pl, s, part, dep, row);
         const uint32_t dst = is_k ? sK + slot * kTile : sV + slot * kTile, bar = bars + 8 * f_bar;
         const CUtensorMap* m = dep ? (is_k ? &maps.kd : &maps.vd) : (is_k ? &maps.k : &maps.v);
+        // A V slot's first depth rows: behind them may be a sequence tile that only the other query tile sees.
+        if (!is_k && dep && pl.dep_rows < kBN && s < pl.n_s + 2) {
+          zero_tails(smem_raw + (2 + KS + slot) * kTile, D / 64, kBN, pl.dep_rows, lane, 32);
+          __syncwarp();
+        }
         if (elect_one()) {
           mbar_expect_tx(bar, dep ? pl.dep_rows * 2 * D : kTile);
           if (dep) tma_load_dep_tile<D>(dst, m, bar, kHalfBytes, h, row, b, dep5);

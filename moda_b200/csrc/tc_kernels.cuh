@@ -362,16 +362,17 @@ __host__ __device__ constexpr uint32_t instr_desc(uint32_t fmt, uint32_t n, bool
 enum BarId : int { kBarQ = 0, kBarK, kBarV, kBarS, kBarP, kBarO, kBarKFree, kBarVFree, kBarCount };
 
 // Depth rows that a tile of `rows` key rows holds: all of them, except for an in-place layer cache, whose
-// TMA boxes are whole positions of L rows.  What a box leaves of the tile is zeros (zero_tails) or
-// stale rows of sequence keys, and its columns are masked.
+// TMA boxes are whole positions of L rows.  What a box leaves of the tile is zeros (zero_tails) or rows of
+// sequence keys that the same query tile has multiplied, and its columns are masked.
 __host__ __device__ __forceinline__ int dep_tile_rows(const Params& p, int rows) {
   return (p.Ls == p.L) ? rows : rows / p.L * p.L;
 }
 // Zeros in the rows [used, rows) of n_boxes consecutive boxes of `rows` rows of 128 bytes: what no box
-// of depth rows fills must not hold an earlier kernel's bytes, since 0 x NaN is NaN in a matmul.
-__device__ __forceinline__ void zero_tails(unsigned char* boxes, int n_boxes, int rows, int used) {
+// of depth rows fills must not hold an earlier kernel's bytes, nor rows that only another query tile has
+// to do with, since 0 x NaN is NaN in a matmul.  Threads first, first + step, ..
+__device__ __forceinline__ void zero_tails(unsigned char* boxes, int n_boxes, int rows, int used, int first, int step) {
   const int per = (rows - used) * 8;
-  for (int i = threadIdx.x; i < n_boxes * per; i += blockDim.x)
+  for (int i = first; i < n_boxes * per; i += step)
     *reinterpret_cast<uint4*>(boxes + ((i / per) * rows + used) * 128 + (i % per) * 16) = make_uint4(0, 0, 0, 0);
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
 }
@@ -460,7 +461,7 @@ fwd_kernel(const __grid_constant__ Params p, const __grid_constant__ FwdMaps map
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   }
-  if (walk.n_dep > 0 && dep_rows < kBN) zero_tails(gbase + 2 * kTile, D / 64, kBN, dep_rows);   // V
+  if (walk.n_dep > 0 && dep_rows < kBN) zero_tails(gbase + 2 * kTile, D / 64, kBN, dep_rows, tid, blockDim.x);   // V
   if (warp == 0) {
     tmem_alloc(ctl + 64, 256);
     tmem_relinquish();

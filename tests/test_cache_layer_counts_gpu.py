@@ -50,3 +50,23 @@ def test_layer_count(built_library, T, G, L, cap, mode, D):
         err, size = (a - b).norm(dim=-1), b.norm(dim=-1)          # row by row: none missing, none foreign
         assert (err <= 2e-2 * (size + size.mean()) + 1e-3).all(), name
     assert M.device_status() == 0
+
+
+@pytest.mark.parametrize("D", [64, 128])
+def test_a_later_sequence_row_that_is_not_finite(built_library, D):
+    """Two query tiles share the forward's V slots: what the second one's sequence tile leaves behind a depth
+    tile that does not fill its slot is not multiplied into the first one's rows.  L = 33: depth tiles of 99
+    rows, 43 of them for the first query tile (rows 256..383) and 37 for the second (384..493), so that the
+    first meets both slots after the key tile of positions 384..493."""
+    import moda_b200 as M
+    B, T, H, L, dt = 10, 494, 8, 33, torch.bfloat16
+    gen = torch.Generator(device="cuda").manual_seed(D)
+    mk = lambda: torch.randn(B, T, H, D, generator=gen, device="cuda", dtype=dt)  # noqa: E731
+    q, k, v = mk(), mk(), mk()
+    cache = M.DepthKVCache(B, T, L + 1, H, D, dt, "cuda")
+    for _ in range(L):
+        cache.append(mk(), mk())
+    clean = cache.attend(q, k, v, chunk_visible=True)
+    v[:, 384 + 105] = float("inf")
+    dirty = cache.attend(q, k, v, chunk_visible=True)
+    assert torch.equal(clean[:, :384], dirty[:, :384])
