@@ -108,7 +108,11 @@ inline cudaError_t launch_bwd(const Params& p, const BwdMaps& m, const BwdBuffer
   // The ends of a launch are a share of it that shrinks with the CTAs an SM works through: 12-layer stack of
   // B = 2, T = 2048, H = 4, G = 4 (512 CTAs of dq) 3.79 -> 3.64 ms, B = 3, T = 1531, H = 5, G = 2 (360) 234 -> 220 us,
   // T = 65536, G = 8, H = 8 (32768) 187.6 and 188.1 ms.
-  const bool overlap = !fused && (int64_t)((p.T_q + kBM - 1) / kBM) * p.H * p.B <= (int64_t)16 * n_sm;
+  // A caller may have the key gradients written over the keys: every key tile is read by the CTA that writes its
+  // gradient and, before that, by dq, which must then have ended.
+  auto over = [](const View& out, const View& a, const View& b) { return out.ptr != nullptr && (out.ptr == a.ptr || out.ptr == b.ptr); };
+  const bool in_place = over(p.dk, p.k, p.v) || over(p.dv, p.k, p.v) || over(p.dkd, p.kd, p.vd) || over(p.dvd, p.kd, p.vd);
+  const bool overlap = !fused && !in_place && (int64_t)((p.T_q + kBM - 1) / kBM) * p.H * p.B <= (int64_t)16 * n_sm;
   if (fused) {
     if constexpr (D == 128) {
       if ((e = cudaMemsetAsync(w.kvmax, 0, w.kvmax_bytes, st)) != cudaSuccess) return e;
