@@ -21,9 +21,9 @@
 //    instructions, as many as on fp32 FMAs).  The backward's gradient rows take the place of the K
 //    and V rows of their stage and leave by TMA too.
 // Against the fp32-FMA kernels these replace: B = 256, T = 197, H = 6, D = 64, L = 11: forward 0.356 ->
-// 0.168 ms, backward 0.479 -> 0.298 ms (6.2 of the measured 6.56 TB/s copy bandwidth); D = 128, L = 32, G = 1 (53 GB):
-// 8.53 -> 7.90 ms; B = 2, T = 4093, H = 4, G = 4, D = 128, L = 24: 0.241 -> 0.085 ms and, against the
-// attention-tile mma.sync kernels, 0.520 -> 0.149 ms.
+// 0.166 ms, backward 0.479 -> 0.312 ms (6.0 of the measured 6.5 TB/s copy bandwidth); D = 128, L = 32, G = 1 (53 GB):
+// 8.53 -> 7.93 ms; B = 2, T = 4093, H = 4, G = 4, D = 128, L = 24: 0.241 -> 0.077 ms and, against the
+// attention-tile mma.sync kernels, 0.520 -> 0.150 ms.
 //
 // Lane layout: g = lane >> 2, t = lane & 3.  A chunk is 16 bytes = 8 channels of a row.
 //  * K (and q, dO; V for dO V^T): lane (g, t) takes chunks t, t + 4, .. of row g.  Word w of chunk
@@ -34,9 +34,18 @@
 //  * An 8 x 8 transpose (movmatrix) of the words of the first layout gives the right operand with
 //    the query rows as the contracted index, for channels 32 j + 8 t + 2 w, + 1 of the result: a lane's
 //    results of the four words are one 16-byte chunk.
-// P and dS enter as two 16-bit numbers each, the value and what its rounding left over (2^-17 relative
-// for bf16), not as one: the probabilities keep the precision they have as fp32 numbers next to
-// 16-bit K, V and results.
+// P and dS enter as the sum of 16-bit numbers, so that what they have beyond 16 bits is not lost: three
+// (split3), which hold all 24 bits of the fp32 value, or in the backward at G > 4 two (split2, 2^-18
+// relative for bf16); in fp16, whose range is smaller, after a power of two has been taken out
+// (Scaled).  With up to four query rows the parts take the other four columns (rows, where the queries
+// are the contracted index) of the same instructions: query q has columns 2 q, 2 q + 1, whose scores
+// come out twice, and the results of the two are added in the end.  Scores are summed in fp32 outside
+// the matrix unit, which cuts its running sum at every step.
+// Against 64 bits (q of 1/4, 1 and 4, dO of 1e-5..64, L = 1..64, G = 1..8, both head dims) the errors of o, dq, dk
+// and dv are then those of the fp32-FMA kernels to 1e-5 of themselves, and values that are not the rounded
+// exact one as few (o in bf16 1.0e-4, 1.2e-4 with FMAs); lse errs by 4.5e-8 (bf16) and 5.0e-8 (fp16), 5.0e-8
+// and 4.9e-8 with FMAs.  (Two parts for all and sums in the matrix unit: 1.4e-3 of o; in fp16 gradients of dO =
+// 1e-5 up to eight times the error, and NaN where scale dS passed 65504.)
 #pragma once
 #include "common.cuh"
 #include "simt_mma_kernels.cuh"
@@ -67,12 +76,67 @@ __device__ __forceinline__ uint32_t transpose8x8(uint32_t x) {
   asm volatile("movmatrix.sync.aligned.m8n8.trans.b16 %0, %1;" : "=r"(y) : "r"(x));
   return y;
 }
-// (a, b) as a 16-bit pair and the pair of what the rounding left over
-template <typename T> __device__ __forceinline__ void split_pair(float a, float b, uint32_t& hi, uint32_t& lo) {
+// (a, b) cut to 16 bits each.
+template <typename T> __device__ __forceinline__ uint32_t cut_pair(float a, float b);
+template <> __device__ __forceinline__ uint32_t cut_pair<__nv_bfloat16>(float a, float b) {
+  return __byte_perm(__float_as_uint(a), __float_as_uint(b), 0x7632u);
+}
+template <> __device__ __forceinline__ uint32_t cut_pair<__half>(float a, float b) {
+  uint32_t w;
+  asm("cvt.rz.f16x2.f32 %0, %1, %2;" : "=r"(w) : "f"(b), "f"(a));
+  return w;
+}
+// (a, b) as the sum of three 16-bit pairs: the value cut to 8 (bf16) or 11 (fp16) bits, what that left over cut
+// again, and the rest.  2^-30 of the value keeps the later parts from being zero, which have the sign of
+// the first one, so that P V is infinite, and not NaN, where a row of V is.
+template <typename T> __device__ __forceinline__ void split3(float a, float b, uint32_t (&w)[3]) {
+  constexpr float kKeep = 0x1p-30f;
+  w[0] = cut_pair<T>(a, b);
+  const float2 x = Pack<T>::unpack(w[0]);
+  const float a1 = fmaf(a, kKeep, a - x.x), b1 = fmaf(b, kKeep, b - x.y);
+  w[1] = cut_pair<T>(a1, b1);
+  const float2 y = Pack<T>::unpack(w[1]);
+  w[2] = cut_pair<T>(fmaf(a, kKeep, a1 - y.x), fmaf(b, kKeep, b1 - y.y));
+}
+// (a, b) rounded to 16 bits, and what the rounding left over.
+template <typename T> __device__ __forceinline__ void split2(float a, float b, uint32_t& hi, uint32_t& lo) {
   hi = Pack<T>::pack(a, b);
   const float2 h = Pack<T>::unpack(hi);
   lo = Pack<T>::pack(a - h.x, b - h.y);
 }
+// At most four query rows, contracted index = depth rows: the operand words of a pair of them.  The first column of
+// a query holds parts 0 and 2, its second part 1 and nothing more (2^-30, as above).
+template <typename T> __device__ __forceinline__ void split3_columns(float a, float b, bool second, uint32_t& w0, uint32_t& w1) {
+  uint32_t w[3];
+  split3<T>(a, b, w);
+  w0 = second ? w[1] : w[0];
+  w1 = second ? cut_pair<T>(a * 0x1p-30f, b * 0x1p-30f) : w[2];
+}
+// The same, contracted index = queries: the words of one query's two indexes.
+template <typename T> __device__ __forceinline__ float cut(float a) { return Pack<T>::unpack(cut_pair<T>(a, 0.f)).x; }
+template <typename T> __device__ __forceinline__ void split3_rows(float a, uint32_t& w0, uint32_t& w1) {
+  const float h = cut<T>(a), r = a - h, m = cut<T>(r);
+  w0 = cut_pair<T>(h, m);
+  w1 = cut_pair<T>(r - m, 0.f);
+}
+// What a fp16 operand holds of fp32 values: those of a warp's step times the power of two that takes their
+// largest magnitude to [2^14, 2^15), so that none overflows and the smallest step left is 2^-38 of the
+// largest (times 65504 that is less than the smallest fp16 result).  bf16 has the range of fp32.
+template <typename T> struct Scaled {
+  float up = 1.f, down = 1.f;
+  static constexpr bool kUsed = std::is_same<T, __half>::value;
+  __device__ __forceinline__ Scaled(float a, float b, float c, float d) {
+    if constexpr (kUsed) {
+      const float m = fmaxf(fmaxf(fabsf(a), fabsf(b)), fmaxf(fabsf(c), fabsf(d)));
+      const uint32_t e = min(240u, 268u - (__reduce_max_sync(0xffffffffu, __float_as_uint(m)) >> 23));
+      up = __uint_as_float(e << 23);
+      down = __uint_as_float((254u - e) << 23);
+    }
+  }
+};
+constexpr float kUpP = 0x1p15f, kDownP = 0x1p-15f;     // the same for probabilities, which are at most 1
+template <typename T> __device__ __forceinline__ constexpr float up_p() { return Scaled<T>::kUsed ? kUpP : 1.f; }
+template <typename T> __device__ __forceinline__ constexpr float down_p() { return Scaled<T>::kUsed ? kDownP : 1.f; }
 __device__ __forceinline__ float quad_sum(float x) {
   x += __shfl_xor_sync(0xffffffffu, x, 1);
   return x + __shfl_xor_sync(0xffffffffu, x, 2);
@@ -232,12 +296,12 @@ template <int D> __device__ __forceinline__ uint4 query_chunk(const unsigned cha
 }
 
 // acc[i] += (rows of `tile`)^T x: for 64 channels of a tile (box i) the 8 channels of chunk g as left
-// operands, each made from the tile rows of operand columns 2 t, 2 t + 1 (+ 8), and the pair x of
-// right operands (16-bit values and what their rounding left over).  Result [e][c]: channel 8 g + e
-// of query 2 t + c.  `left` rows of the tile exist (kAll: all, or the others are zeros).
-template <typename T, bool kAll>
+// operands, each made from the tile rows of operand columns 2 t, 2 t + 1 (+ 8), and the N parts of x
+// as right operands, x = their sum times `down`.  Result [e][c]: channel 8 g + e of query 2 t + c.
+// `left` rows of the tile exist (kAll: all, or the others are zeros).
+template <typename T, bool kAll, bool kScaled, int N>
 __device__ __forceinline__ void add_transposed(float (&acc)[8][2], const unsigned char* tile, int i, int g, int t4, int left,
-                                               const uint32_t (&hi)[2], const uint32_t (&lo)[2]) {
+                                               const uint32_t (&x0)[N], const uint32_t (&x1)[N], float down) {
   uint32_t w[4][4];
 #pragma unroll
   for (int x = 0; x < 4; ++x) {                     // a row that does not exist is whatever the stage held before
@@ -249,10 +313,15 @@ __device__ __forceinline__ void add_transposed(float (&acc)[8][2], const unsigne
   for (int e = 0; e < 4; ++e) {                     // channels 2 e (rows g of the operand) and 2 e + 1 (rows g + 8)
     const uint32_t a[4] = {__byte_perm(w[0][e], w[1][e], 0x5410u), __byte_perm(w[0][e], w[1][e], 0x7632u),
                            __byte_perm(w[2][e], w[3][e], 0x5410u), __byte_perm(w[2][e], w[3][e], 0x7632u)};
-    float c[4] = {acc[2 * e][0], acc[2 * e][1], acc[2 * e + 1][0], acc[2 * e + 1][1]};
-    simt::Mma<T>::run(c, a, hi[0], hi[1]);
-    simt::Mma<T>::run(c, a, lo[0], lo[1]);
-    acc[2 * e][0] = c[0]; acc[2 * e][1] = c[1]; acc[2 * e + 1][0] = c[2]; acc[2 * e + 1][1] = c[3];
+    float c[4] = {0.f, 0.f, 0.f, 0.f};
+    if (!kScaled) { c[0] = acc[2 * e][0]; c[1] = acc[2 * e][1]; c[2] = acc[2 * e + 1][0]; c[3] = acc[2 * e + 1][1]; }
+#pragma unroll
+    for (int part = N - 1; part >= 0; --part) simt::Mma<T>::run(c, a, x0[part], x1[part]);
+#pragma unroll
+    for (int x = 0; x < 4; ++x) {
+      float& r = acc[2 * e + (x >> 1)][x & 1];
+      r = kScaled ? fmaf(c[x], down, r) : c[x];
+    }
   }
 }
 
@@ -265,8 +334,9 @@ template <int D, int NQ, int NT> __device__ __forceinline__ void zero_tiles(cons
 }
 
 // ------------------------------------------------------------------------- forward
-template <typename T, int D, bool kOne>
-__global__ void __launch_bounds__(kWarps * 32, D == 64 ? 6 : 3) fwd_kernel(const __grid_constant__ Params p, const __grid_constant__ Maps maps) {
+// QR: query rows that a step has columns for, 4 (G <= 4) or 8.
+template <typename T, int D, bool kOne, int QR>
+__global__ void __launch_bounds__(kWarps * 32, D == 64 ? (kOne ? 6 : 5) : 3) fwd_kernel(const __grid_constant__ Params p, const __grid_constant__ Maps maps) {
   constexpr int J = D / 32, I = D / 64;
   extern __shared__ __align__(1024) unsigned char smem[];
   if (smem_u32(smem) & 1023u) {                     // the swizzle is a function of the shared-memory address
@@ -276,6 +346,7 @@ __global__ void __launch_bounds__(kWarps * 32, D == 64 ? 6 : 3) fwd_kernel(const
   if (tc::launch_failed(p)) return;
   const int lane = threadIdx.x & 31, g = lane >> 2, t4 = lane & 3;
   const int my_row = row_of(g >> 1, g & 1);         // tile row (+ 8 nt) of this lane's K operand
+  const int my_q = QR == 4 ? g >> 1 : g;            // query of this lane's scores
   Ring<D, 1> ring(p, smem);
   if (kOne) zero_tiles(ring);
   const Stride stride(p, gridDim.x * kWarps);
@@ -293,26 +364,26 @@ __global__ void __launch_bounds__(kWarps * 32, D == 64 ? 6 : 3) fwd_kernel(const
     const bool first = kOne || s.l0 == 0;
     if (first) {
 #pragma unroll
-      for (int j = 0; j < J; ++j) qa[j] = g < n_rows ? query_chunk<D>(ring.queries, g, t4 + 4 * j) : make_uint4(0, 0, 0, 0);
+      for (int j = 0; j < J; ++j) qa[j] = my_q < n_rows ? query_chunk<D>(ring.queries, my_q, t4 + 4 * j) : make_uint4(0, 0, 0, 0);
     }
     __syncwarp();                                   // the other stage and the query rows have been read
     if (next.b < p.B) ring.issue(p, maps, nullptr, next);
     const unsigned char *kt = ring.stage(), *vt = kt + tile_bytes<D>();
     const int left = p.L - s.l0;                    // rows of the tile that exist (16 or more: all)
 
-    float pv[4];                                    // scores of query g; columns 2 t, 2 t + 1, 8 + 2 t, 8 + 2 t + 1
+    float pv[4];                                    // scores of my_q; columns 2 t, 2 t + 1, 8 + 2 t, 8 + 2 t + 1
 #pragma unroll
     for (int nt = 0; nt < 2; ++nt) {
-      float sc[4] = {0.f, 0.f, 0.f, 0.f};           // [2], [3] stay 0
 #pragma unroll
       for (int j = 0; j < J; ++j) {
         const uint4 kw = tile_chunk<kRows>(kt, 8 * nt + my_row, t4 + 4 * j);
         const uint32_t a0[4] = {qa[j].x, 0u, qa[j].y, 0u}, a1[4] = {qa[j].z, 0u, qa[j].w, 0u};
-        simt::Mma<T>::run(sc, a0, kw.x, kw.y);
-        simt::Mma<T>::run(sc, a1, kw.z, kw.w);
+        float s0[4] = {0.f, 0.f, 0.f, 0.f}, s1[4] = {0.f, 0.f, 0.f, 0.f};           // [2], [3] stay 0
+        simt::Mma<T>::run(s0, a0, kw.x, kw.y);
+        simt::Mma<T>::run(s1, a1, kw.z, kw.w);
+        pv[2 * nt] = j == 0 ? s0[0] + s1[0] : pv[2 * nt] + (s0[0] + s1[0]);
+        pv[2 * nt + 1] = j == 0 ? s0[1] + s1[1] : pv[2 * nt + 1] + (s0[1] + s1[1]);
       }
-      pv[2 * nt] = sc[0];
-      pv[2 * nt + 1] = sc[1];
     }
     float bm = -INFINITY;
 #pragma unroll
@@ -330,7 +401,7 @@ __global__ void __launch_bounds__(kWarps * 32, D == 64 ? 6 : 3) fwd_kernel(const
     float total = 0.f;
     if (kOne) {
       total = quad_sum(part);
-      const float inv = 1.f / total;
+      const float inv = up_p<T>() / total;
 #pragma unroll
       for (int x = 0; x < 4; ++x) pv[x] *= inv;
     }
@@ -349,33 +420,44 @@ __global__ void __launch_bounds__(kWarps * 32, D == 64 ? 6 : 3) fwd_kernel(const
 #pragma unroll
         for (int e = 0; e < 8; ++e) { acc[i][e][0] *= a0; acc[i][e][1] *= a1; }
     }
-    uint32_t ph[2], pl[2];
-    split_pair<T>(pv[0], pv[1], ph[0], pl[0]);
-    split_pair<T>(pv[2], pv[3], ph[1], pl[1]);
+    if (!kOne && Scaled<T>::kUsed) {
 #pragma unroll
-    for (int i = 0; i < I; ++i) add_transposed<T, kOne>(acc[i], vt, i, g, t4, left, ph, pl);
+      for (int x = 0; x < 4; ++x) pv[x] *= kUpP;
+    }
+    constexpr int N = QR == 4 ? 2 : 3;
+    uint32_t p0[N], p1[N];
+    if constexpr (QR == 4) {
+      split3_columns<T>(pv[0], pv[1], g & 1, p0[0], p0[1]);
+      split3_columns<T>(pv[2], pv[3], g & 1, p1[0], p1[1]);
+    } else {
+      split3<T>(pv[0], pv[1], p0);
+      split3<T>(pv[2], pv[3], p1);
+    }
+#pragma unroll
+    for (int i = 0; i < I; ++i) add_transposed<T, kOne, false>(acc[i], vt, i, g, t4, left, p0, p1, 1.f);
 
     if (kOne || left <= kRows) {
       const int r = s.t * p.G + s.g0;
       float inv[2] = {1.f, 1.f};
       if (!kOne) {
         total = quad_sum(lsum);
-        const float v = 1.f / total;
+        const float v = down_p<T>() / total;
         inv[0] = __shfl_sync(0xffffffffu, v, 8 * t4);
         inv[1] = __shfl_sync(0xffffffffu, v, 8 * t4 + 4);
       }
-      T* op = reinterpret_cast<T*>(p.o.ptr) + p.o.off(s.b, r + 2 * t4, s.h) + 8 * g;
+      constexpr int NC = QR == 4 ? 1 : 2;           // query rows that a lane ends with
+      T* op = reinterpret_cast<T*>(p.o.ptr) + p.o.off(s.b, r + NC * t4, s.h) + 8 * g;
 #pragma unroll
-      for (int c = 0; c < 2; ++c)
-        if (2 * t4 + c < n_rows)
+      for (int c = 0; c < NC; ++c)
+        if (NC * t4 + c < n_rows)
 #pragma unroll
           for (int i = 0; i < I; ++i) {
             float f[8];
 #pragma unroll
-            for (int e = 0; e < 8; ++e) f[e] = kOne ? acc[i][e][c] : acc[i][e][c] * inv[c];
+            for (int e = 0; e < 8; ++e) f[e] = (QR == 4 ? acc[i][e][0] + acc[i][e][1] : acc[i][e][c]) * (kOne ? down_p<T>() : inv[c]);
             *reinterpret_cast<uint4*>(op + c * p.o.st + 64 * i) = pack8<T>(f);
           }
-      if (t4 == 0 && g < n_rows) p.lse[((int64_t)s.b * p.T_q + r + g) * p.H + s.h] = m + log2f(total);
+      if (t4 == 0 && my_q < n_rows && (QR == 8 || (g & 1) == 0)) p.lse[((int64_t)s.b * p.T_q + r + my_q) * p.H + s.h] = m + log2f(total);
     }
     s = next;
   }
@@ -389,8 +471,8 @@ __global__ void __launch_bounds__(kWarps * 32, D == 64 ? 6 : 3) fwd_kernel(const
 // G <= 8: the query rows of a position are one group.  Scores are computed transposed (K as the left
 // operand: 16 depth rows at once), so that P^T and dS^T are left operands of dV = P^T dO and
 // dK = dS^T Q as they come.
-template <typename T, int D, bool kOne, bool kAdd>
-__global__ void __launch_bounds__(kWarps * 32, D == 64 ? (kAdd ? 3 : kOne ? 5 : 4) : 3) bwd_kernel(const __grid_constant__ Params p, const __grid_constant__ Maps maps, const __grid_constant__ OutMaps omaps) {
+template <typename T, int D, bool kOne, bool kAdd, int QR>
+__global__ void __launch_bounds__(kWarps * 32, D == 64 ? (kAdd ? 3 : 4) : 3) bwd_kernel(const __grid_constant__ Params p, const __grid_constant__ Maps maps, const __grid_constant__ OutMaps omaps) {
   constexpr int J = D / 32, I = D / 64;
   extern __shared__ __align__(1024) unsigned char smem[];
   if (smem_u32(smem) & 1023u) {
@@ -400,24 +482,26 @@ __global__ void __launch_bounds__(kWarps * 32, D == 64 ? (kAdd ? 3 : kOne ? 5 : 
   if (tc::launch_failed(p)) return;
   const int lane = threadIdx.x & 31, g = lane >> 2, t4 = lane & 3;
   const int my_row = row_of(g >> 1, g & 1);         // tile row (+ 8) of this lane's operands and results
-  const bool row_ok = g < p.G;
+  constexpr int NC = QR == 4 ? 1 : 2;               // queries of a lane's two columns
+  const int my_q = QR == 4 ? g >> 1 : g, q0 = NC * t4;       // query of this lane's rows; first query of its columns
+  const bool row_ok = my_q < p.G;
   constexpr int NT = bwd_tiles<D, kAdd>();
   Ring<D, 3, NT> ring(p, smem);
   if (kOne) zero_tiles(ring);
   const Stride stride(p, gridDim.x * kWarps);
   Step s = first_step(p);
   uint4 qa[J], da[J];
-  float delta[2] = {0.f, 0.f}, lse[2] = {0.f, 0.f};          // of queries 2 t, 2 t + 1
+  float delta[2] = {0.f, 0.f}, lse[2] = {0.f, 0.f};          // of queries q0 (NC = 2: and q0 + 1)
   float lse_next[2] = {INFINITY, INFINITY};                  // P of a query that does not exist: exp2(-inf) = 0
   float dq[I][8][2];                                         // [channel 8 (g + 8 i) + e][query 2 t + c]
   bool ok = true;
   auto issue = [&](const Step& x) {
     ring.issue(p, maps, &omaps, x);
     if (kOne || x.l0 == 0) {
-      const float* l = p.lse + ((int64_t)x.b * p.T_q + x.t * p.G + 2 * t4) * p.H + x.h;
+      const float* l = p.lse + ((int64_t)x.b * p.T_q + x.t * p.G + q0) * p.H + x.h;
 #pragma unroll
-      for (int c = 0; c < 2; ++c)
-        if (2 * t4 + c < p.G) lse_next[c] = l[c * p.H];
+      for (int c = 0; c < NC; ++c)
+        if (q0 + c < p.G) lse_next[c] = l[c * p.H];
     }
   };
   if (s.b < p.B) issue(s);
@@ -432,9 +516,9 @@ __global__ void __launch_bounds__(kWarps * 32, D == 64 ? (kAdd ? 3 : kOne ? 5 : 
 #pragma unroll
       for (int j = 0; j < J; ++j) {
         const uint4 zero = make_uint4(0, 0, 0, 0);
-        qa[j] = row_ok ? query_chunk<D>(ring.queries, g, t4 + 4 * j) : zero;
-        da[j] = row_ok ? query_chunk<D>(ring.queries + p.G * 2 * D, g, t4 + 4 * j) : zero;
-        const uint4 oa = row_ok ? query_chunk<D>(ring.queries + 2 * p.G * 2 * D, g, t4 + 4 * j) : zero;
+        qa[j] = row_ok ? query_chunk<D>(ring.queries, my_q, t4 + 4 * j) : zero;
+        da[j] = row_ok ? query_chunk<D>(ring.queries + p.G * 2 * D, my_q, t4 + 4 * j) : zero;
+        const uint4 oa = row_ok ? query_chunk<D>(ring.queries + 2 * p.G * 2 * D, my_q, t4 + 4 * j) : zero;
         float of[8], df[8];
         unpack8<T>(oa, of);
         unpack8<T>(da[j], df);
@@ -443,7 +527,7 @@ __global__ void __launch_bounds__(kWarps * 32, D == 64 ? (kAdd ? 3 : kOne ? 5 : 
       }
       dl = quad_sum(dl);
       delta[0] = __shfl_sync(0xffffffffu, dl, 8 * t4);
-      delta[1] = __shfl_sync(0xffffffffu, dl, 8 * t4 + 4);
+      if (NC == 2) delta[1] = __shfl_sync(0xffffffffu, dl, 8 * t4 + 4);
 #pragma unroll
       for (int i = 0; i < I; ++i)
 #pragma unroll
@@ -454,38 +538,52 @@ __global__ void __launch_bounds__(kWarps * 32, D == 64 ? (kAdd ? 3 : kOne ? 5 : 
     const unsigned char *kt = ring.stage(), *vt = kt + tile_bytes<D>();
     const int left = p.L - s.l0;                    // rows of the tile that exist (16 or more: all)
 
-    // S^T and dP^T: [2 nt + c] = (tile row my_row + 8 nt, query 2 t + c)
-    float sc[4] = {0.f, 0.f, 0.f, 0.f}, dp[4] = {0.f, 0.f, 0.f, 0.f};
+    // S^T and dP^T: [2 nt + c] = (tile row my_row + 8 nt, query q0 + c)
+    float sc[4], dp[4];
 #pragma unroll
     for (int j = 0; j < J; ++j) {
       const uint4 k0 = tile_chunk<kRows>(kt, my_row, t4 + 4 * j), k1 = tile_chunk<kRows>(kt, 8 + my_row, t4 + 4 * j);
       const uint32_t ka[4] = {k0.x, k1.x, k0.y, k1.y}, kb[4] = {k0.z, k1.z, k0.w, k1.w};
-      simt::Mma<T>::run(sc, ka, qa[j].x, qa[j].y);
-      simt::Mma<T>::run(sc, kb, qa[j].z, qa[j].w);
+      float s0[4] = {0.f, 0.f, 0.f, 0.f}, d0[4] = {0.f, 0.f, 0.f, 0.f};
+      simt::Mma<T>::run(s0, ka, qa[j].x, qa[j].y);
+      simt::Mma<T>::run(s0, kb, qa[j].z, qa[j].w);
       const uint4 v0 = tile_chunk<kRows>(vt, my_row, t4 + 4 * j), v1 = tile_chunk<kRows>(vt, 8 + my_row, t4 + 4 * j);
       const uint32_t va[4] = {v0.x, v1.x, v0.y, v1.y}, vb[4] = {v0.z, v1.z, v0.w, v1.w};
-      simt::Mma<T>::run(dp, va, da[j].x, da[j].y);
-      simt::Mma<T>::run(dp, vb, da[j].z, da[j].w);
+      simt::Mma<T>::run(d0, va, da[j].x, da[j].y);
+      simt::Mma<T>::run(d0, vb, da[j].z, da[j].w);
+#pragma unroll
+      for (int x = 0; x < 4; ++x) {
+        sc[x] = j == 0 ? s0[x] : sc[x] + s0[x];
+        dp[x] = j == 0 ? d0[x] : dp[x] + d0[x];
+      }
     }
-    // left operands P^T and scale dS^T: rows my_row, my_row + 8; contracted index = queries, then the
-    // queries again with what the rounding left over
-    uint32_t pt[4], dt[4];
+    // left operands P^T and scale dS^T: rows my_row, my_row + 8; contracted index = queries, twice
+    float pw[2][NC], ds[2][NC];
 #pragma unroll
     for (int nt = 0; nt < 2; ++nt) {
       const bool live = my_row + 8 * nt < left;
-      float pw[2], ds[2];
 #pragma unroll
-      for (int c = 0; c < 2; ++c) {
-        pw[c] = live ? fast_exp2(fmaf(sc[2 * nt + c], p.scale_log2, -lse[c])) : 0.f;
-        ds[c] = live ? pw[c] * (dp[2 * nt + c] - delta[c]) * p.scale : 0.f;
+      for (int c = 0; c < NC; ++c) {
+        pw[nt][c] = live ? fast_exp2(fmaf(sc[2 * nt + c], p.scale_log2, -lse[c])) : 0.f;
+        ds[nt][c] = live ? pw[nt][c] * (dp[2 * nt + c] - delta[c]) * p.scale : 0.f;
       }
-      split_pair<T>(pw[0], pw[1], pt[nt], pt[nt + 2]);
-      split_pair<T>(ds[0], ds[1], dt[nt], dt[nt + 2]);
+    }
+    const Scaled<T> ps(pw[0][0], pw[1][0], pw[0][NC - 1], pw[1][NC - 1]), dss(ds[0][0], ds[1][0], ds[0][NC - 1], ds[1][NC - 1]);
+    uint32_t pt[4], dt[4];
+#pragma unroll
+    for (int nt = 0; nt < 2; ++nt) {
+      if constexpr (QR == 4) {
+        split3_rows<T>(pw[nt][0] * ps.up, pt[nt], pt[nt + 2]);
+        split3_rows<T>(ds[nt][0] * dss.up, dt[nt], dt[nt + 2]);
+      } else {
+        split2<T>(pw[nt][0] * ps.up, pw[nt][1] * ps.up, pt[nt], pt[nt + 2]);
+        split2<T>(ds[nt][0] * dss.up, ds[nt][1] * dss.up, dt[nt], dt[nt + 2]);
+      }
     }
     {   // dQ^T += K^T (scale dS)^T
-      const uint32_t hi[2] = {transpose8x8(dt[0]), transpose8x8(dt[1])}, lo[2] = {transpose8x8(dt[2]), transpose8x8(dt[3])};
+      const uint32_t d0[2] = {transpose8x8(dt[0]), transpose8x8(dt[2])}, d1[2] = {transpose8x8(dt[1]), transpose8x8(dt[3])};
 #pragma unroll
-      for (int i = 0; i < I; ++i) add_transposed<T, kOne>(dq[i], kt, i, g, t4, left, hi, lo);
+      for (int i = 0; i < I; ++i) add_transposed<T, kOne, Scaled<T>::kUsed>(dq[i], kt, i, g, t4, left, d0, d1, dss.down);
     }
     // The gradient rows take the place of the K and V rows and leave as a tile: stored from registers, a
     // lane's 16 bytes beside three others', every instruction would write half lines.
@@ -505,8 +603,8 @@ __global__ void __launch_bounds__(kWarps * 32, D == 64 ? (kAdd ? 3 : kOne ? 5 : 
         simt::Mma<T>::run(cv, pt, db, db);
 #pragma unroll
         for (int x = 0; x < 4; ++x) {
-          gk[x >> 1][2 * w + (x & 1)] = ck[x];
-          gv[x >> 1][2 * w + (x & 1)] = cv[x];
+          gk[x >> 1][2 * w + (x & 1)] = ck[x] * dss.down;
+          gv[x >> 1][2 * w + (x & 1)] = cv[x] * ps.down;
         }
       }
 #pragma unroll
@@ -528,15 +626,15 @@ __global__ void __launch_bounds__(kWarps * 32, D == 64 ? (kAdd ? 3 : kOne ? 5 : 
     ring.store(p, omaps, s);
 
     if (kOne || left <= kRows) {
-      T* qp = reinterpret_cast<T*>(p.dq.ptr) + p.dq.off(s.b, s.t * p.G + 2 * t4, s.h) + 8 * g;
+      T* qp = reinterpret_cast<T*>(p.dq.ptr) + p.dq.off(s.b, s.t * p.G + q0, s.h) + 8 * g;
 #pragma unroll
-      for (int c = 0; c < 2; ++c)
-        if (2 * t4 + c < p.G)
+      for (int c = 0; c < NC; ++c)
+        if (q0 + c < p.G)
 #pragma unroll
           for (int i = 0; i < I; ++i) {
             float f[8];
 #pragma unroll
-            for (int e = 0; e < 8; ++e) f[e] = dq[i][e][c];
+            for (int e = 0; e < 8; ++e) f[e] = QR == 4 ? dq[i][e][0] + dq[i][e][1] : dq[i][e][c];
             *reinterpret_cast<uint4*>(qp + c * p.dq.st + 64 * i) = pack8<T>(f);
           }
     }

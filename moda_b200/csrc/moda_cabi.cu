@@ -227,18 +227,22 @@ int fda_launch(K kernel, int id, size_t smem, int n_sm, cudaStream_t st, const P
   g_last_launches += 1;
   return MODA_OK;
 }
-template <typename T, int D, bool kOne>
+template <typename T, int D, bool kOne, int QR>
 int fda_run(const Params& p, const fda::Maps& maps, const fda::OutMaps& omaps, bool is_bwd, int n_sm, cudaStream_t st) {
-  if (!is_bwd) return fda_launch(fda::fwd_kernel<T, D, kOne>, prof::kFdaFwd, fda::smem_bytes<D, 1>(p.G), n_sm, st, p, maps);
+  if (!is_bwd) return fda_launch(fda::fwd_kernel<T, D, kOne, QR>, prof::kFdaFwd, fda::smem_bytes<D, 1>(p.G), n_sm, st, p, maps);
   if (p.acc_depth)
-    return fda_launch(fda::bwd_kernel<T, D, kOne, true>, prof::kFdaBwd, fda::smem_bytes<D, 3, fda::bwd_tiles<D, true>()>(p.G), n_sm, st, p, maps, omaps);
-  return fda_launch(fda::bwd_kernel<T, D, kOne, false>, prof::kFdaBwd, fda::smem_bytes<D, 3>(p.G), n_sm, st, p, maps, omaps);
+    return fda_launch(fda::bwd_kernel<T, D, kOne, true, QR>, prof::kFdaBwd, fda::smem_bytes<D, 3, fda::bwd_tiles<D, true>()>(p.G), n_sm, st, p, maps, omaps);
+  return fda_launch(fda::bwd_kernel<T, D, kOne, false, QR>, prof::kFdaBwd, fda::smem_bytes<D, 3>(p.G), n_sm, st, p, maps, omaps);
+}
+template <typename T, int D>
+int fda_run_l(const Params& p, const fda::Maps& m, const fda::OutMaps& om, bool is_bwd, int n_sm, cudaStream_t st) {
+  if (p.L <= fda::kRows)
+    return p.G <= 4 ? fda_run<T, D, true, 4>(p, m, om, is_bwd, n_sm, st) : fda_run<T, D, true, 8>(p, m, om, is_bwd, n_sm, st);
+  return p.G <= 4 ? fda_run<T, D, false, 4>(p, m, om, is_bwd, n_sm, st) : fda_run<T, D, false, 8>(p, m, om, is_bwd, n_sm, st);
 }
 template <typename T>
 int fda_run_d(const Params& p, const fda::Maps& m, const fda::OutMaps& om, int D, bool is_bwd, int n_sm, cudaStream_t st) {
-  const bool one = p.L <= fda::kRows;
-  if (D == 64) return one ? fda_run<T, 64, true>(p, m, om, is_bwd, n_sm, st) : fda_run<T, 64, false>(p, m, om, is_bwd, n_sm, st);
-  return one ? fda_run<T, 128, true>(p, m, om, is_bwd, n_sm, st) : fda_run<T, 128, false>(p, m, om, is_bwd, n_sm, st);
+  return D == 64 ? fda_run_l<T, 64>(p, m, om, is_bwd, n_sm, st) : fda_run_l<T, 128>(p, m, om, is_bwd, n_sm, st);
 }
 int fda_dispatch(const Params& p, const moda_problem* prob, bool is_bwd, int n_sm, cudaStream_t st) {
   fda::Maps maps;
