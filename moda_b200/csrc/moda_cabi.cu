@@ -280,13 +280,29 @@ int tc_forward(const Params& p, const moda_problem* prob, int n_sm, cudaStream_t
   return tc::fwd(p, prob, st, &g_last_launches, &g_last_cuda_error);
 }
 
-// Short sequences take the one-CTA-per-head backward where its kernel has a CTA for the whole problem: 256
-// keys are what 16 warps hold in registers at D = 64, and 512 query rows keep it from being longer than the
-// tile kernels, whose matrix instructions are faster (T = 197, 256 heads or more: 351 us against 404).
-bool use_short_bwd(const moda_problem* att) {
-  return att->path == MODA_PATH_AUTO && att->mode != MODA_DEPTH_ONLY && att->D == shortseq::kD && att->L == 0 &&
-         att->T_kv <= shortseq::kMaxKeys && (int64_t)att->T_kv * att->G <= 2 * shortseq::kMaxKeys &&
-         (int64_t)att->B * att->H <= 0x7fffffff;
+// Short sequences take the one-CTA-per-head backward where its kernel has a CTA for the whole problem (256
+// keys are what 16 warps hold in registers at D = 64; 512 query rows) and enough heads: a head is a serial
+// chain on one SM, which the tile kernels divide.  Estimates in us for 148 SMs, fitted to 22 shapes
+// (T = 32..256, G = 1..8, causal and all keys) with 1 to 512 heads each:
+//   one round of CTAs  5 + blocks of 32 query rows x (2.2 + 0.07 warps, at least 8 / warps), under a causal
+//                      mask 0.01 of it less a warp, CTAs that share an SM a quarter longer
+//   tile kernels       8 + heads x (0.065 query tiles + 0.04 key tiles), at least 12 + 0.4 blocks
+// Short against tile kernels, causal, G = 1: T = 64 from 1 head 10.6, 12.2, 256 heads 13, 29; T = 197 1 head 25, 15, 64 heads
+// 25, 22, 128 heads 25, 35, 192 heads 46, 49, 512 heads 92, 114; T = 256, G = 2: 1 head 50, 19, 128 heads 51, 55,
+// 256 heads 103, 101.
+bool use_short_bwd(const moda_problem* att, int n_sm) {
+  if (!(att->path == MODA_PATH_AUTO && att->mode != MODA_DEPTH_ONLY && att->D == shortseq::kD && att->L == 0 &&
+        att->T_kv <= shortseq::kMaxKeys && (int64_t)att->T_kv * att->G <= 2 * shortseq::kMaxKeys && (int64_t)att->B * att->H <= 0x7fffffff))
+    return false;
+  const int warps = (att->T_kv + 15) / 16, T_q = att->T_kv * att->G, blocks = (T_q + shortseq::kBQ - 1) / shortseq::kBQ;
+  const int64_t heads = (int64_t)att->B * att->H;
+  const int64_t per_sm = std::min<int64_t>((227 << 10) / shortseq::smem_bytes(warps), 16 / warps);      // 128 registers a thread
+  const int64_t rounds = (heads + n_sm * per_sm - 1) / (n_sm * per_sm);
+  double round_us = 5 + blocks * std::max(2.2 + 0.07 * warps, 8.0 / warps);
+  if (att->mode != MODA_NONCAUSAL) round_us *= 1 - 0.01 * warps;
+  if (per_sm > 1 && heads > n_sm) round_us *= 1.25;
+  const double per_head = (0.065 * ((T_q + 127) / 128) + 0.04 * ((att->T_kv + 127) / 128)) * 148 / n_sm;
+  return 2 + rounds * round_us < std::max(12 + 0.4 * blocks, 8 + heads * per_head);
 }
 template <typename T>
 int short_bwd(const Params& p, cudaStream_t st) {
@@ -487,7 +503,7 @@ int moda_b200_bwd(const moda_problem* prob, const moda_tensor4* q, const moda_te
     if (int rc = fda_dispatch(p, prob, true, n_sm, st)) return rc;
     p = sequence_part(p);
   }
-  if (path == MODA_PATH_TCGEN05 && use_short_bwd(&att))
+  if (path == MODA_PATH_TCGEN05 && use_short_bwd(&att, n_sm))
     return prob->dtype == MODA_BF16 ? short_bwd<__nv_bfloat16>(p, st) : short_bwd<__half>(p, st);
   if (path == MODA_PATH_TCGEN05) {
     void* extra = reinterpret_cast<unsigned char*>(workspace) + delta_bytes(prob);

@@ -16,8 +16,9 @@
 // block i + 2 (cp.async) and the row sums delta = o . dO of block i + 1 are made during block i, which
 // takes the statistics launch and its pass over o and dO away.
 // What bounds it now is the rate of the warp-level matrix instructions (about 8 clocks of an SM each), which
-// is why it has no advantage beyond a few hundred keys.  B = 256, T = 197, H = 6: statistics + dq + dk/dv
-// 404 us -> 351 us; B = 64: 122 -> 97 us a layer.
+// is why it has no advantage beyond a few hundred keys, and the serial chain of a head's query blocks, which
+// is why it has none with few heads (use_short_bwd).  1536 heads (B = 256, H = 6), T = 197: statistics + dq +
+// dk/dv 404 us -> 351 us; 384 heads: 122 -> 97 us a layer.
 #pragma once
 #include "simt_mma_kernels.cuh"
 
