@@ -10,6 +10,7 @@
 // tc_bwd_fused_kernel.cuh), which is why it is not the default.
 #pragma once
 #include <algorithm>
+#include <functional>
 
 #include "tc_bwd_fused_kernel.cuh"
 
@@ -52,21 +53,63 @@ struct BwdBuffers { float *delta_t, *lse_t, *norm_t; float4* scale_blk; int* kvm
 
 // CTAs that share a key tile of the dk/dv kernel.  A tile's query steps are a serial chain on one SM and
 // under a causal mask the first tile has twice the average: with few tiles the launch lasts as long as
-// that one.  Estimate in steps of 64 query rows, per CTA kFixed more (set-up, first loads, the sums' way
-// through the cluster, the stores and the SMs that pairs leave idle): the longest CTA, or all of them
-// over the SMs; a split has to win a tenth.  D = 128: B = 2, T = 2048, H = 4, G = 4 (128 tiles): two CTAs 116 -> 81 us;
-// B = 3, T = 1531, H = 5, G = 2 (180 tiles): two CTAs 67 -> 85 us, so one; kFixed = 20 puts both right.
-inline int dkv_parts(const Params& p, int n_sm) {
-  constexpr double kFixed = 20;
-  const double tiles = (double)((p.T_kv + kBN - 1) / kBN) * p.H * p.B;
-  const double longest = (p.T_q + kStep - 1) / kStep, all = tiles * longest * (p.mode == kNonCausal ? 1.0 : 0.5);
-  double best = std::max(longest + kFixed, (all + tiles * kFixed) / n_sm);
+// that one.  But dk/dv's CTAs also run beside dq's, and shares that find no free SM at once cost more than they save.
+// So the two grids are dealt out to the SMs as the GPU does it, heaviest CTA first, and the split whose last
+// CTA ends first is taken if it wins a twentieth (beside the depth-gradient grid, which the deal leaves out:
+// three).  In steps of 64 query rows x 128 keys a CTA takes its steps (dq's, of 64 keys, 0.7 each) and a fixed
+// part: 15 for dq, 20 for dk/dv (set-up, first loads, stores), 3 more in a cluster (the sums' way through it);
+// clusters of two and four find room on 95 and 87 % of the SMs.  344 shapes (2..320 tiles, D = 64 and 128, both types,
+// three modes) with one, two and four CTAs a tile timed each: the choice is 0.7 % off the best on average, and
+// slower than one CTA by more than 4 % (5 %) at one; dk/dv looked at as if it had the GPU to itself is 5 % off, and
+// slower, by up to 39 %, at 61.
+// D = 128, causal, us with one, two, four: T = 1024, G = 1: H = 4 30, 25, 35, H = 12 36, 42, 72; T = 4096, G = 2, H = 2 115, 70, 88.
+struct SplitShape { int n_sm, T_kv, G, heads, causal, beside_dq, beside_depth; };
+inline bool operator==(const SplitShape& a, const SplitShape& b) {
+  return a.n_sm == b.n_sm && a.T_kv == b.T_kv && a.G == b.G && a.heads == b.heads && a.causal == b.causal && a.beside_dq == b.beside_dq &&
+         a.beside_depth == b.beside_depth;
+}
+constexpr int kSplitSms = 512;
+inline double last_cta_end(const SplitShape& s, int parts) {
+  constexpr double kDqStep = 0.7, kDqFixed = 15, kFixed = 20, kCluster = 3;
+  double free_at[kSplitSms] = {0.};                         // a heap, the SM that is free first on top
+  const int n_sm = parts == 1 ? s.n_sm : parts == 2 ? s.n_sm * 95 / 100 : s.n_sm * 87 / 100;
+  double end = 0;
+  auto deal = [&](int tiles, double steps, double fixed, int n) {
+    for (int i = 0; i < tiles; ++i) {
+      const double cost = fixed + steps * (s.causal ? 1. - (double)i / tiles : 1.);
+      for (int h = 0; h < s.heads; ++h) {
+        for (int k = 0; k < n; ++k) std::pop_heap(free_at, free_at + n_sm - k, std::greater<double>());
+        const double t = free_at[n_sm - n] + cost;          // from when the last of the n SMs is free
+        for (int k = n - 1; k >= 0; --k) {
+          free_at[n_sm - 1 - k] = t;
+          std::push_heap(free_at, free_at + n_sm - k, std::greater<double>());
+        }
+        end = std::max(end, t);
+      }
+    }
+  };
+  const int64_t T_q = (int64_t)s.T_kv * s.G, q_tiles = (T_q + kBM - 1) / kBM, q_steps = (T_q + kStep - 1) / kStep;
+  // dq with more than two CTAs an SM ends on all SMs at about the same time
+  if (s.beside_dq && q_tiles * s.heads <= 2 * s.n_sm) deal((int)q_tiles, kDqStep * ((s.T_kv + kStep - 1) / kStep), kDqFixed, 1);
+  deal((s.T_kv + kBN - 1) / kBN, (double)q_steps / parts, kFixed + (parts > 1 ? kCluster : 0), parts);
+  return end;
+}
+inline int dkv_parts(const Params& p, int n_sm, bool beside_dq, bool beside_depth) {
+  const int64_t tiles = (int64_t)((p.T_kv + kBN - 1) / kBN) * p.H * p.B, steps = (p.T_q + kStep - 1) / kStep;
+  if (tiles > 2 * n_sm || steps < 4 || n_sm < 8 || n_sm > kSplitSms) return 1;
+  const SplitShape shape{n_sm, p.T_kv, p.G, p.H * p.B, p.mode != kNonCausal, beside_dq, beside_depth};
+  // The deal takes some 30 us of host time, and its answer depends on the shape alone: a thread keeps a few.
+  static thread_local struct { SplitShape shape; int parts; } known[16];       // parts 0: empty
+  auto& slot = known[((uint32_t)p.T_kv * 31u + (uint32_t)p.G * 7u + (uint32_t)shape.heads) & 15u];
+  if (slot.parts != 0 && slot.shape == shape) return slot.parts;
+  double best = last_cta_end(shape, 1);
   int parts = 1;
-  for (int n = 2; n <= 4; n *= 2) {
-    if (longest < 2 * n) break;
-    const double t = std::max(longest / n + kFixed, (all + n * tiles * kFixed) / n_sm);
-    if (t < 0.9 * best) { best = t; parts = n; }
+  for (int n = 2; n <= 4 && steps >= 2 * n; n *= 2) {
+    const double t = last_cta_end(shape, n);
+    if (t < (beside_depth ? 0.85 : 0.95) * best) { best = t; parts = n; }
   }
+  slot.shape = shape;
+  slot.parts = parts;
   return parts;
 }
 
@@ -105,9 +148,9 @@ inline cudaError_t launch_bwd(const Params& p, const BwdMaps& m, const BwdBuffer
   float* lse_t = w.lse_t;
   const int n_seq = (p.T_kv + kBN - 1) / kBN;
   const int n_dep_tiles = (int)(((int64_t)p.T_kv * p.L + kBN - 1) / kBN);
-  // The ends of a launch are a share of it that shrinks with the CTAs an SM works through: 12-layer stack of
-  // B = 2, T = 2048, H = 4, G = 4 (512 CTAs of dq) 3.79 -> 3.64 ms, B = 3, T = 1531, H = 5, G = 2 (360) 234 -> 220 us,
-  // T = 65536, G = 8, H = 8 (32768) 187.6 and 188.1 ms.
+  // The ends of a launch are a share of it that shrinks with the CTAs an SM works through.  Backward with overlap
+  // against without (causal, all keys, chunk-visible, D = 64 and 128): 0.80-0.94 at one or two CTAs of dq an SM,
+  // 0.94-0.98 at 3.5, 0.97-0.99 at 7, 0.98-1.01 at 14, 0.95-1.08 and no tendency at 28 and 42.
   // A caller may have the key gradients written over the keys: every key tile is read by the CTA that writes its
   // gradient and, before that, by dq, which must then have ended.
   auto over = [](const View& out, const View& a, const View& b) { return out.ptr != nullptr && (out.ptr == a.ptr || out.ptr == b.ptr); };
@@ -187,11 +230,11 @@ inline cudaError_t launch_bwd(const Params& p, const BwdMaps& m, const BwdBuffer
     *launches += 1;
     {
       const bool own_tiles = !dg && n_dep_tiles > 0;
-      const int parts = own_tiles ? 1 : dkv_parts(p, n_sm);
+      const int parts = own_tiles ? 1 : dkv_parts(p, n_sm, overlap, overlap && dg);
       auto kern = parts > 1 ? dkv_kernel<T, D, true> : dkv_kernel<T, D, false>;
       if ((e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dkv_smem)) != cudaSuccess) return e;
       const dim3 grid((n_seq + (own_tiles ? n_dep_tiles : 0)) * parts, p.H, p.B);
-      prof::Scope ps(prof::kDkvTc, st);
+      prof::Scope ps(parts > 1 ? prof::kDkvSplitTc : prof::kDkvTc, st);
       e = launch_next(kern, grid, kDkvThreads, dkv_smem, parts, overlap, st, p, m.dkv, (const float*)delta_t, (const float*)lse_t, T_qp, n_seq);
     }
     if (e != cudaSuccess) return e;

@@ -123,8 +123,8 @@ def _failing_backward(wt, B, T, H, D):
 
 
 @pytest.mark.parametrize("D", [64, 128])
-@pytest.mark.parametrize("B,T,H", [(1, 512, 1),        # dk/dv: four tiles of two CTAs each
-                                   (1, 1024, 2),       # of four
+@pytest.mark.parametrize("B,T,H", [(1, 512, 1),        # dk/dv: four tiles of four CTAs each
+                                   (1, 1024, 4),       # 32 of two
                                    (8, 128, 32)])      # more CTAs than SMs, no clusters
 def test_failed_backward_with_clusters(built_library, B, T, H, D):
     """CTAs that share a key tile leave together when their waits run out, and store nothing."""
