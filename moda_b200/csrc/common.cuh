@@ -41,7 +41,7 @@ struct Params {
   // overwriting (every depth row has one owning thread block, so this stays deterministic).
   int Ls;
   int acc_depth;
-  int launch_id;                    // number of the call, never 0
+  int launch_id;                    // number of the call; 0: a captured one
 };
 
 // Memory row of depth row c (see Params::Ls).

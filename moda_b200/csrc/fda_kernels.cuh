@@ -215,6 +215,7 @@ struct Ring {
   uint32_t bars;
   volatile int* abort_flag;
   int issued = 0, taken = 0;           // steps issued / taken so far
+  bool failed;                         // the call has, before this block began
   __device__ __forceinline__ Ring(const Params& p, unsigned char* smem) {
     const int w = threadIdx.x >> 5;
     const uint32_t q_bytes = NQ * min(p.G, 8) * 2 * D;
@@ -230,7 +231,7 @@ struct Ring {
       asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     }
-    __syncthreads();
+    failed = __syncthreads_or(tc::failure_seen(p)) != 0;
   }
   // Loads of step s; a unit's first step brings the query rows.
   __device__ __forceinline__ void issue(const Params& p, const Maps& maps, const OutMaps* grads, const Step& s) {
@@ -343,11 +344,11 @@ __global__ void __launch_bounds__(kWarps * 32, D == 64 ? (kOne ? 6 : 5) : 3) fwd
     if (threadIdx.x == 0) tc::record_failure(2 << 8);
     return;
   }
-  if (tc::launch_failed(p)) return;
   const int lane = threadIdx.x & 31, g = lane >> 2, t4 = lane & 3;
   const int my_row = row_of(g >> 1, g & 1);         // tile row (+ 8 nt) of this lane's K operand
   const int my_q = QR == 4 ? g >> 1 : g;            // query of this lane's scores
   Ring<D, 1> ring(p, smem);
+  if (ring.failed) return;
   if (kOne) zero_tiles(ring);
   const Stride stride(p, gridDim.x * kWarps);
   Step s = first_step(p);
@@ -479,7 +480,6 @@ __global__ void __launch_bounds__(kWarps * 32, D == 64 ? (kAdd ? 3 : 4) : 3) bwd
     if (threadIdx.x == 0) tc::record_failure(2 << 8);
     return;
   }
-  if (tc::launch_failed(p)) return;
   const int lane = threadIdx.x & 31, g = lane >> 2, t4 = lane & 3;
   const int my_row = row_of(g >> 1, g & 1);         // tile row (+ 8) of this lane's operands and results
   constexpr int NC = QR == 4 ? 1 : 2;               // queries of a lane's two columns
@@ -487,6 +487,7 @@ __global__ void __launch_bounds__(kWarps * 32, D == 64 ? (kAdd ? 3 : 4) : 3) bwd
   const bool row_ok = my_q < p.G;
   constexpr int NT = bwd_tiles<D, kAdd>();
   Ring<D, 3, NT> ring(p, smem);
+  if (ring.failed) return;
   if (kOne) zero_tiles(ring);
   const Stride stride(p, gridDim.x * kWarps);
   Step s = first_step(p);

@@ -165,7 +165,7 @@ bwd_fused_kernel(const __grid_constant__ Params p, const __grid_constant__ DkvMa
   volatile int* drain_flag = reinterpret_cast<volatile int*>(gctl + 8 * kMaxBars + 8);
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  if (launch_failed(p)) return;
+  const bool seen = failure_seen(p);
 
   const int h = blockIdx.y, b = blockIdx.z;
   const int c0 = (int)blockIdx.x * kBN;        // key tile 0 is seen by every query row: heaviest tiles first
@@ -199,9 +199,13 @@ bwd_fused_kernel(const __grid_constant__ Params p, const __grid_constant__ DkvMa
     tmem_relinquish();
   }
   tc_fence_before();
-  __syncthreads();
+  const bool leave = __syncthreads_or(seen) != 0;
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
+  if (leave) {
+    if (warp == 0) tmem_dealloc(tmem, 512);
+    return;
+  }
   const uint32_t tmem_S = tmem, tmem_P = tmem + 64, tmem_dV = tmem + 128, tmem_dK = tmem + 256;
   const uint32_t tmem_V = tmem + 384, tmem_dQ = tmem + 448;
   constexpr uint32_t fmt = std::is_same<T, __nv_bfloat16>::value ? 1u : 0u;

@@ -224,7 +224,7 @@ dq_kernel(const __grid_constant__ Params p, const __grid_constant__ DqMaps maps,
   volatile int* drain_flag = reinterpret_cast<volatile int*>(gctl + 8 * kMaxBars + 8);
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  if (launch_failed(p)) { grid_before(); return; }
+  const bool seen = failure_seen(p);
 
   const int n_qt = (p.T_q + kBM - 1) / kBM;
   const BlockId bid = block_order(p, D);
@@ -273,11 +273,13 @@ dq_kernel(const __grid_constant__ Params p, const __grid_constant__ DqMaps maps,
     tmem_relinquish();
   }
   tc_fence_before();
-  __syncthreads();
+  const bool leave = __syncthreads_or(seen) != 0;
   tc_fence_after();
-  grid_before();
-  grid_started();
   const uint32_t tmem = *tmem_slot;
+  if (leave && warp == 0) tmem_dealloc(tmem, 512);
+  grid_before();
+  if (leave) return;
+  grid_started();
   const uint32_t tmem_dQ = tmem + 256, tmem_Q = tmem + 384, tmem_dO = tmem + 448;
   constexpr uint32_t fmt = std::is_same<T, __nv_bfloat16>::value ? 1u : 0u;
 
@@ -579,7 +581,7 @@ dkv_kernel(const __grid_constant__ Params p, const __grid_constant__ DkvMaps map
   volatile int* peer_failed = reinterpret_cast<volatile int*>(gctl + 8 * kMaxBars + 12);
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  if (!kSplit && launch_failed(p)) { grid_before(); return; }   // (a cluster stays together: below)
+  const bool seen = failure_seen(p);
   const int parts = kSplit ? (int)cluster_size() : 1, part = kSplit ? (int)cluster_rank() : 0;
 
   grid_started();
@@ -619,7 +621,7 @@ dkv_kernel(const __grid_constant__ Params p, const __grid_constant__ DkvMaps map
       mbar_init(bars + 8 * (B_.p0 + i), 128);
       mbar_init(bars + 8 * (B_.r0 + i), 128); mbar_init(bars + 8 * (B_.t0 + i), 1);
     }
-    *abort_flag = kSplit && failure_published(p) ? 1 : 0;
+    *abort_flag = kSplit && seen ? 1 : 0;        // a cluster stays together: its waits end at once
     *drain_flag = 0;
     if (kSplit) *peer_failed = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -630,9 +632,14 @@ dkv_kernel(const __grid_constant__ Params p, const __grid_constant__ DkvMaps map
     tmem_relinquish();
   }
   tc_fence_before();
-  __syncthreads();
+  const bool leave = __syncthreads_or(!kSplit && seen) != 0;
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
+  if (leave) {
+    if (warp == 0) tmem_dealloc(tmem, 512);
+    grid_before();
+    return;
+  }
   const uint32_t tmem_S = tmem, tmem_P = tmem + 64, tmem_dV = tmem + 128, tmem_dK = tmem + 256;
   const uint32_t tmem_K = tmem + 384, tmem_V = tmem + 448;
   constexpr uint32_t fmt = std::is_same<T, __nv_bfloat16>::value ? 1u : 0u;
@@ -1022,7 +1029,7 @@ depth_grad_kernel(const __grid_constant__ Params p, const __grid_constant__ DkvM
   volatile int* drain_flag = reinterpret_cast<volatile int*>(gctl + 112);
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  if (launch_failed(p)) { grid_before(); return; }
+  const bool seen = failure_seen(p);
 
   const int n_xb = (p.T_q + kStep - 1) / kStep;
   const int total = n_xb * p.H * p.B;                   // 64-row blocks; this CTA takes blockIdx.x, + gridDim.x, ...
@@ -1049,9 +1056,14 @@ depth_grad_kernel(const __grid_constant__ Params p, const __grid_constant__ DkvM
     tmem_relinquish();
   }
   tc_fence_before();
-  __syncthreads();
+  const bool leave = __syncthreads_or(seen) != 0;
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
+  if (leave) {
+    if (warp == 0) tmem_dealloc(tmem, 512);
+    grid_before();
+    return;
+  }
   const uint32_t tmem_dV = tmem + 256, tmem_dK = tmem + 384;   // score stage s: tmem + 128 s (+ 64 for dP^T)
   constexpr uint32_t fmt = std::is_same<T, __nv_bfloat16>::value ? 1u : 0u;
 

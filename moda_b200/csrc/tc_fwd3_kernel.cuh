@@ -142,7 +142,7 @@ fwd3_kernel(const __grid_constant__ Params p, const __grid_constant__ Fwd3Maps m
   volatile int* drain_flag = reinterpret_cast<volatile int*>(gctl + 8 * kMaxBars + 8);
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  if (launch_failed(p)) return;
+  const bool seen = failure_seen(p);
 
   const int n_pairs = (p.T_q + 2 * kBM - 1) / (2 * kBM);
   const BlockId bid = block_order(p, D);
@@ -171,14 +171,19 @@ fwd3_kernel(const __grid_constant__ Params p, const __grid_constant__ Fwd3Maps m
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   }
+  if (pl.n > pl.n_s && pl.dep_rows < kBN) zero_tails(smem_raw + (2 + KS) * kTile, 2 * (D / 64), kBN, pl.dep_rows, tid, blockDim.x);   // V
   if (warp == 0) {
     tmem_alloc(bars + 8 * kMaxBars, 512);
     tmem_relinquish();
   }
   tc_fence_before();
-  __syncthreads();
+  const bool leave = __syncthreads_or(seen) != 0;
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
+  if (leave) {
+    if (warp == 0) tmem_dealloc(tmem, 512);
+    return;
+  }
   constexpr uint32_t fmt = std::is_same<T, __nv_bfloat16>::value ? 1u : 0u;
 
   // Warpgroup-wide register reallocation, first thing in every role: all four warps of the last
@@ -208,11 +213,6 @@ fwd3_kernel(const __grid_constant__ Params p, const __grid_constant__ Fwd3Maps m
         f3_step(pl, s, part, dep, row);
         const uint32_t dst = is_k ? sK + slot * kTile : sV + slot * kTile, bar = bars + 8 * f_bar;
         const CUtensorMap* m = dep ? (is_k ? &maps.kd : &maps.vd) : (is_k ? &maps.k : &maps.v);
-        // A V slot's first depth rows: behind them may be a sequence tile that only the other query tile sees.
-        if (!is_k && dep && pl.dep_rows < kBN && s < pl.n_s + 2) {
-          zero_tails(smem_raw + (2 + KS + slot) * kTile, D / 64, kBN, pl.dep_rows, lane, 32);
-          __syncwarp();
-        }
         if (elect_one()) {
           mbar_expect_tx(bar, dep ? pl.dep_rows * 2 * D : kTile);
           if (dep) tma_load_dep_tile<D>(dst, m, bar, kHalfBytes, h, row, b, dep5);
@@ -223,9 +223,23 @@ fwd3_kernel(const __grid_constant__ Params p, const __grid_constant__ Fwd3Maps m
         return true;
       };
       for (int s = 0; ok && s < kLead && s < pl.n; ++s) ok = load(s, true);
-      for (int s = 0; ok && s < pl.n; ++s) {
-        if (s + kLead < pl.n) ok = load(s + kLead, true);
-        if (ok) ok = load(s, false);
+      // What depth tiles that do not fill their V slot leave of it are rows of the last sequence tile there.  The
+      // slot of a sequence tile that only the second query tile has in range is the first one's for the
+      // first time when the second has no depth step left, and is cleared of them then.  (A branch in `load`
+      // costs every call 1 % at T = 4096.)
+      const bool foreign = pl.dep_rows < kBN && pl.w[0].n_seq < pl.w[1].n_seq && pl.w[0].n_dep > pl.w[1].n_dep + 1;
+      int stop = foreign ? pl.n_s + 2 * pl.w[1].n_dep + 1 : pl.n;
+      for (int s = 0;;) {
+        for (; ok && s < stop; ++s) {
+          if (s + kLead < pl.n) ok = load(s + kLead, true);
+          if (ok) ok = load(s, false);
+        }
+        if (!ok || stop == pl.n) break;
+        stop = pl.n;
+        const int slot = s & 1, e_bar = B_::emptyv0 + slot;
+        if (!(ok = s < 2 || mbar_wait(bars + 8 * e_bar, ((s >> 1) - 1) & 1, abort_flag, e_bar))) break;
+        zero_tails(smem_raw + (2 + KS + slot) * kTile, D / 64, kBN, pl.dep_rows, lane, 32);
+        __syncwarp();
       }
       if (!ok) {   // let loads in flight land before the CTA's shared memory is released
         mbar_wait(bars + 8 * B_::q, 0, drain_flag, B_::q);

@@ -51,8 +51,8 @@ template <int D> __host__ __device__ constexpr uint32_t tile_bytes() { return (u
 
 // g_tc_failed is the number (Params::launch_id) of the call in which a wait expired last, written by the
 // CTA's teardown: CTAs of that call's launches which start later return at once, and other calls,
-// whose numbers differ, need nothing cleared before they are enqueued (a captured call, whose number stays,
-// clears the word in its graph).  g_tc_sticky keeps the first
+// whose numbers differ, need nothing cleared before they are enqueued.  A captured call has no number
+// (0): it would keep it, and a failed replay would end every later one.  g_tc_sticky keeps the first
 // failure of any launch, (code << 8) | barrier id of the wait that expired, until the host reads it
 // (moda_b200_device_status), so that a later call cannot erase it.
 __device__ int g_tc_failed;
@@ -62,17 +62,14 @@ __device__ __forceinline__ void record_failure(int code) {
   atomicCAS(&g_tc_sticky, 0, code);
 }
 
-__device__ __forceinline__ bool failure_published(const Params& p) {
-  return *reinterpret_cast<volatile int*>(&g_tc_failed) == p.launch_id;
-}
-// One answer for the whole CTA, from all of its threads: the word may change between two threads' loads, and
-// a warp that leaves in part, or a CTA without some of its warps, breaks the collectives and
-// arrival counts of those that stay.
-__device__ __forceinline__ bool launch_failed(const Params& p) {
-  return __syncthreads_or(threadIdx.x == 0 && failure_published(p)) != 0;
+// Whether the call has failed, for thread 0 alone: the CTA leaves as a whole or not at all, by what its set-up
+// barrier makes of it.  (The word may change between two threads' loads, and a warp that leaves in part, or a
+// CTA without some of its warps, breaks the collectives and arrival counts of those that stay.)
+__device__ __forceinline__ bool failure_seen(const Params& p) {
+  return threadIdx.x == 0 && p.launch_id != 0 && *reinterpret_cast<volatile int*>(&g_tc_failed) == p.launch_id;
 }
 __device__ __forceinline__ void publish_failure(const Params& p, volatile int* abort_flag) {
-  if (*abort_flag != 0) atomicExch(&g_tc_failed, p.launch_id);
+  if (*abort_flag != 0 && p.launch_id != 0) atomicExch(&g_tc_failed, p.launch_id);
 }
 
 struct FwdMaps { CUtensorMap q, k, v, kd, vd; };
@@ -436,7 +433,7 @@ fwd_kernel(const __grid_constant__ Params p, const __grid_constant__ FwdMaps map
   volatile int* drain_flag = reinterpret_cast<volatile int*>(gctl + 76);   // never set: lets the drain waits run
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  if (launch_failed(p)) return;   // an earlier CTA failed: do nothing
+  const bool seen = failure_seen(p);   // an earlier CTA failed: do nothing
 
   const int n_qt = (p.T_q + kBM - 1) / kBM;
   const BlockId bid = block_order(p, D);
@@ -467,9 +464,13 @@ fwd_kernel(const __grid_constant__ Params p, const __grid_constant__ FwdMaps map
     tmem_relinquish();
   }
   tc_fence_before();
-  __syncthreads();
+  const bool leave = __syncthreads_or(seen) != 0;
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
+  if (leave) {
+    if (warp == 0) tmem_dealloc(tmem, 256);
+    return;
+  }
   const uint32_t tmem_S = tmem, tmem_O = tmem + 128;
   constexpr uint32_t fmt = std::is_same<T, __nv_bfloat16>::value ? 1u : 0u;
 

@@ -223,8 +223,8 @@ def test_expired_wait_in_the_backward_is_reported_and_context_survives(built_lib
 
 @pytest.mark.parametrize("bwd", [False, True])
 def test_a_captured_call_runs_again_after_a_failure(built_library, bwd):
-    """The call's number is part of the graph: what a replay left there does not stop the next one, which here
-    waits for the limit again."""
+    """A failed replay does not stop the next one, which here waits for the limit again (the call's number would
+    be part of the graph)."""
     from moda_b200 import _cabi
     wt = _wait_test_library()
     B, T, H, D = 1, 64, 1, 128
