@@ -224,14 +224,15 @@ struct Ring {
     unsigned char* ctl = smem + kWarps * (2 * kStage + q_bytes);
     bars = smem_u32(ctl) + w * 16;
     abort_flag = reinterpret_cast<volatile int*>(ctl + kWarps * 16);     // abort, drain
-    if (threadIdx.x == 0) abort_flag[0] = abort_flag[1] = 0;
+    if (threadIdx.x == 0) { abort_flag[0] = 0; abort_flag[1] = tc::failure_seen(p) ? 1 : 0; }
     if ((threadIdx.x & 31) == 0) {
       tc::mbar_init(bars, 1);
       tc::mbar_init(bars + 8, 1);
       asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     }
-    failed = __syncthreads_or(tc::failure_seen(p)) != 0;
+    __syncthreads();
+    failed = abort_flag[1] != 0;
   }
   // Loads of step s; a unit's first step brings the query rows.
   __device__ __forceinline__ void issue(const Params& p, const Maps& maps, const OutMaps* grads, const Step& s) {

@@ -190,7 +190,7 @@ bwd_fused_kernel(const __grid_constant__ Params p, const __grid_constant__ DkvMa
       mbar_init(bars + 8 * (B_::qd0 + i), 1);
     }
     *abort_flag = 0;
-    *drain_flag = 0;
+    *drain_flag = seen ? 1 : 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   }
@@ -199,8 +199,9 @@ bwd_fused_kernel(const __grid_constant__ Params p, const __grid_constant__ DkvMa
     tmem_relinquish();
   }
   tc_fence_before();
-  const bool leave = __syncthreads_or(seen) != 0;
+  __syncthreads();
   tc_fence_after();
+  const bool leave = *drain_flag != 0;
   const uint32_t tmem = *tmem_slot;
   if (leave) {
     if (warp == 0) tmem_dealloc(tmem, 512);

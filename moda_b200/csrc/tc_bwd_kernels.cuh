@@ -263,7 +263,7 @@ dq_kernel(const __grid_constant__ Params p, const __grid_constant__ DqMaps maps,
       mbar_init(bars + 8 * (B_.r0 + i), 128); mbar_init(bars + 8 * (B_.t0 + i), 1);
     }
     *abort_flag = 0;
-    *drain_flag = 0;
+    *drain_flag = seen ? 1 : 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   }
@@ -273,12 +273,14 @@ dq_kernel(const __grid_constant__ Params p, const __grid_constant__ DqMaps maps,
     tmem_relinquish();
   }
   tc_fence_before();
-  const bool leave = __syncthreads_or(seen) != 0;
+  __syncthreads();
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
-  if (leave && warp == 0) tmem_dealloc(tmem, 512);
   grid_before();
-  if (leave) return;
+  if (*drain_flag != 0) {
+    if (warp == 0) tmem_dealloc(tmem, 512);
+    return;
+  }
   grid_started();
   const uint32_t tmem_dQ = tmem + 256, tmem_Q = tmem + 384, tmem_dO = tmem + 448;
   constexpr uint32_t fmt = std::is_same<T, __nv_bfloat16>::value ? 1u : 0u;
@@ -622,7 +624,7 @@ dkv_kernel(const __grid_constant__ Params p, const __grid_constant__ DkvMaps map
       mbar_init(bars + 8 * (B_.r0 + i), 128); mbar_init(bars + 8 * (B_.t0 + i), 1);
     }
     *abort_flag = kSplit && seen ? 1 : 0;        // a cluster stays together: its waits end at once
-    *drain_flag = 0;
+    *drain_flag = !kSplit && seen ? 1 : 0;
     if (kSplit) *peer_failed = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -632,8 +634,9 @@ dkv_kernel(const __grid_constant__ Params p, const __grid_constant__ DkvMaps map
     tmem_relinquish();
   }
   tc_fence_before();
-  const bool leave = __syncthreads_or(!kSplit && seen) != 0;
+  __syncthreads();
   tc_fence_after();
+  const bool leave = !kSplit && *drain_flag != 0;
   const uint32_t tmem = *tmem_slot;
   if (leave) {
     if (warp == 0) tmem_dealloc(tmem, 512);
@@ -1047,7 +1050,7 @@ depth_grad_kernel(const __grid_constant__ Params p, const __grid_constant__ DkvM
     mbar_init(bars + 8 * kDgE, 256);
     mbar_init(bars + 8 * kDgQFree, 1);
     *abort_flag = 0;
-    *drain_flag = 0;
+    *drain_flag = seen ? 1 : 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   }
@@ -1056,8 +1059,9 @@ depth_grad_kernel(const __grid_constant__ Params p, const __grid_constant__ DkvM
     tmem_relinquish();
   }
   tc_fence_before();
-  const bool leave = __syncthreads_or(seen) != 0;
+  __syncthreads();
   tc_fence_after();
+  const bool leave = *drain_flag != 0;
   const uint32_t tmem = *tmem_slot;
   if (leave) {
     if (warp == 0) tmem_dealloc(tmem, 512);

@@ -167,7 +167,7 @@ fwd3_kernel(const __grid_constant__ Params p, const __grid_constant__ Fwd3Maps m
       for (int j = 0; j < kF3Parts; ++j) mbar_init(bars + 8 * (B_::p0 + 2 * j + i), 4);   // one arrival per softmax warp
     }
     *abort_flag = 0;
-    *drain_flag = 0;
+    *drain_flag = seen ? 1 : 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   }
@@ -177,8 +177,9 @@ fwd3_kernel(const __grid_constant__ Params p, const __grid_constant__ Fwd3Maps m
     tmem_relinquish();
   }
   tc_fence_before();
-  const bool leave = __syncthreads_or(seen) != 0;
+  __syncthreads();
   tc_fence_after();
+  const bool leave = *drain_flag != 0;
   const uint32_t tmem = *tmem_slot;
   if (leave) {
     if (warp == 0) tmem_dealloc(tmem, 512);

@@ -62,9 +62,11 @@ __device__ __forceinline__ void record_failure(int code) {
   atomicCAS(&g_tc_sticky, 0, code);
 }
 
-// Whether the call has failed, for thread 0 alone: the CTA leaves as a whole or not at all, by what its set-up
-// barrier makes of it.  (The word may change between two threads' loads, and a warp that leaves in part, or a
-// CTA without some of its warps, breaks the collectives and arrival counts of those that stay.)
+// Whether the call has failed, for thread 0 alone, which hands the answer to the CTA with the other words that it
+// sets up: the CTA leaves as a whole or not at all.  (The word may change between two threads' loads, and a
+// warp that leaves in part, or a CTA without some of its warps, breaks the collectives and arrival counts
+// of those that stay.)  The word it takes is drain_flag, which a CTA that stays never sets: the waits of
+// the drains do not give up.
 __device__ __forceinline__ bool failure_seen(const Params& p) {
   return threadIdx.x == 0 && p.launch_id != 0 && *reinterpret_cast<volatile int*>(&g_tc_failed) == p.launch_id;
 }
@@ -430,7 +432,7 @@ fwd_kernel(const __grid_constant__ Params p, const __grid_constant__ FwdMaps map
   const uint32_t bars = ctl;                                    // kBarCount x 8 bytes
   volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(gctl + 64);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(gctl + 72);
-  volatile int* drain_flag = reinterpret_cast<volatile int*>(gctl + 76);   // never set: lets the drain waits run
+  volatile int* drain_flag = reinterpret_cast<volatile int*>(gctl + 76);
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const bool seen = failure_seen(p);   // an earlier CTA failed: do nothing
@@ -454,7 +456,7 @@ fwd_kernel(const __grid_constant__ Params p, const __grid_constant__ FwdMaps map
     mbar_init(bars + 8 * kBarKFree, 1);
     mbar_init(bars + 8 * kBarVFree, 1);
     *abort_flag = 0;
-    *drain_flag = 0;
+    *drain_flag = seen ? 1 : 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   }
@@ -464,8 +466,9 @@ fwd_kernel(const __grid_constant__ Params p, const __grid_constant__ FwdMaps map
     tmem_relinquish();
   }
   tc_fence_before();
-  const bool leave = __syncthreads_or(seen) != 0;
+  __syncthreads();
   tc_fence_after();
+  const bool leave = *drain_flag != 0;
   const uint32_t tmem = *tmem_slot;
   if (leave) {
     if (warp == 0) tmem_dealloc(tmem, 256);
