@@ -3,6 +3,7 @@ recorded, on one stream, one backward).  Reference: the packed cache rebuilt bef
 (``torch.stack`` of the earlier layers' K/V) through the ordinary operator."""
 import copy
 import pickle
+import time
 
 import pytest
 import torch
@@ -134,3 +135,45 @@ def test_copies_of_a_used_cache(built_library, how, train):
         assert torch.equal(at(other.grad_k), at(cache.grad_k)) and torch.equal(at(other.grad_v), at(cache.grad_v))
     with torch.no_grad():
         assert torch.equal(other.attend(*layers[2], moda_group_num=G), cache.attend(*layers[2], moda_group_num=G))
+
+
+def test_a_deeper_layer_after_an_earlier_one(built_library):
+    """The first attention whose backward runs stores its share of the gradient cache; one that read more layers
+    and comes later (its gradient comes by way of the CPU) finds the slots beyond it cleared."""
+    layers, dout = _leaves(5, 4)
+    leaves = [x for lay in layers for x in lay]
+
+    def grads(outs):
+        last = outs[3].cpu()
+        last.register_hook(lambda g: time.sleep(0.3))
+        for x in leaves:
+            x.grad = None
+        torch.autograd.backward([outs[0], outs[1], outs[2], last], dout[:3] + [dout[3].cpu()])
+        return [x.grad for x in leaves]
+
+    _check(grads(_cached(layers)), grads(_rebuilt(layers)))
+
+
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("causal", [False, True])
+def test_deep_stack(built_library, causal, D):
+    """G = 1, up to 21 cached layers: the bandwidth kernels add gradients in more than one step of a unit."""
+    import moda_b200 as M
+    gen = torch.Generator(device="cuda").manual_seed(D)
+    B, T, H, N = 2, 45, 2, 22
+    mk = lambda: torch.randn(B, T, H, D, generator=gen, device="cuda", dtype=torch.bfloat16).requires_grad_(True)  # noqa: E731
+    layers, dout = [(mk(), mk(), mk()) for _ in range(N)], [mk().detach() for _ in range(N)]
+    leaves = [x for lay in layers for x in lay]
+    cache = M.DepthKVCache(B, T, N + 1, H, D, torch.bfloat16, "cuda")
+    cache.k.fill_(float("nan"))
+    cache.v.fill_(float("nan"))
+    outs, want, kv = [], [], []
+    for i, (q, k, v) in enumerate(layers):
+        outs.append(cache.attend(q, k, v, is_causal=causal))
+        ck, cv = [torch.stack([x[j] for x in kv], dim=2).view(B, T * i, H, D) if kv else None for j in (0, 1)]
+        want.append(M.parallel_moda(q, k, v, cached_k=ck, cached_v=cv, is_causal=causal))
+        cache.append(k, v)
+        kv.append((k, v))
+    assert all(torch.equal(a, b) for a, b in zip(outs, want))
+    _check(torch.autograd.grad(outs, leaves, dout), torch.autograd.grad(want, leaves, dout))
+    assert M.device_status() == 0
