@@ -75,10 +75,11 @@ CHUNK_ROWS = 64
 # L2 by every block and now and then from HBM; dk/dv also re-reads q and dO per key tile).  The
 # depth-gradient kernel (18.3 GB algorithmic) is scaled from its T=8192 capture (1.01 x).
 NCU_TRAFFIC_BYTES = {"tc_fwd": 10.259e9 + 0.744e9, "tc_dq": 11.558e9 + 0.533e9, "tc_dkv": 2.305e9 + 0.263e9,
-                     "tc_depth_grad": 1.01 * 18.3e9, "fda_fwd": 17.72e9, "fda_bwd": 35.43e9}
+                     "tc_depth_grad": 1.01 * 18.3e9, "fda_fwd": 32 * 0.556e9, "fda_bwd": 32 * 1.107e9}
 NCU_TRAFFIC_SOURCE = {"tc_fwd": "one-pass ncu capture of this workload", "tc_dq": "one-pass ncu capture of this workload",
                       "tc_dkv": "one-pass ncu capture of this workload", "tc_depth_grad": "scaled from the T=8192 ncu capture",
-                      "fda_fwd": "ncu capture of this workload", "fda_bwd": "ncu capture of this workload"}
+                      "fda_fwd": "scaled from the small_fda_T8192 ncu capture",
+                      "fda_bwd": "scaled from the small_fda_T8192 ncu capture (writes that stayed in L2 counted)"}
 
 # Algorithmic matmuls (of 2*D*pairs FLOP each) a kernel OWNS - the outputs it alone produces.  The
 # forward owns S and O (2); of the backward's five (S, dP, dV, dK, dQ) the dq kernel owns dQ, the

@@ -100,9 +100,10 @@ __device__ __forceinline__ bool mbar_test(uint32_t bar, uint32_t parity) {
 // The wait sleeps in hardware (mbarrier.try_wait with a suspend-time hint) instead of
 // spinning: a spinning warp takes issue slots from the producer lane and from the softmax
 // warp that shares its SM sub-partition.  Bound: kWaitTries x kWaitHintNs of sleeping.
-// The loop must stay a loop: a kernel has some thirty of these waits, and unrolled (the compiler's
-// choice for a constant trip count) they push the roles' straight-line loops out of the instruction
-// caches (T = 65536, D = 64, G = 8: forward 53.7 -> 48.5 ms, dk/dv 72.1 -> 70.1 ms).
+// The loop must stay a loop: a kernel has some thirty of these waits, and unrolled (the compiler's choice for
+// it as it stands) they push the roles' straight-line loops out of the instruction caches (T = 65536, D = 64,
+// G = 8: forward 53.7 against 48.5 ms, dk/dv 72.1 against 70.1 ms).  Before the failure word had a call's number
+// the compiler kept it a loop by itself: the pragma restores that and is no gain over it.
 __device__ __forceinline__ bool mbar_try(uint32_t bar, uint32_t parity) {
   uint32_t ok;
   asm volatile(
@@ -717,7 +718,8 @@ inline bool make_map_depth(CUtensorMap* m, const View& v, int dtype, const Param
 
 // The tcgen05 kernels take a positive scale (the row maximum is taken before scaling) and, for an
 // in-place layer cache (depth_rows_per_pos > L), at most 64 layers: a position fits the step tile of the
-// smallest pipeline (dq).  A forced path keeps to layer counts that divide 32.
+// smallest pipeline (dq).  A forced path takes the layer counts that it always took, those that divide 32: a
+// caller that forces one asks for a fixed set of kernels, and what was refused stays refused.
 inline bool depth_layout_supported(const moda_problem* pr) {
   if (pr->L == 0 || pr->depth_rows_per_pos <= pr->L || (32 % pr->L) == 0) return true;
   return pr->path == MODA_PATH_AUTO && pr->L <= 64;

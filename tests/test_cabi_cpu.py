@@ -171,7 +171,8 @@ def test_depth_cache_layout_fields_are_validated(lib):
     assert lib.moda_b200_check_problem(r(_prob(L=2, depth_rows_per_pos=11))) == 0
     assert lib.moda_b200_check_problem(r(_prob(L=3, depth_rows_per_pos=2))) == 2     # fewer rows than layers
     assert lib.moda_b200_check_problem(r(_prob(L=2, depth_rows_per_pos=-1))) == 2
-    # the tcgen05 kernels read an in-place cache through 5-D maps only when L divides their 32-row boxes
+    # an in-place cache of a layer count that does not divide 32: not on a forced tcgen05 path, nor (D = 64) for up
+    # to 64 positions
     assert lib.moda_b200_resolve_path(r(_prob(L=4, depth_rows_per_pos=11, G=2, T_kv=64)), 0) == 2
     assert lib.moda_b200_resolve_path(r(_prob(L=3, depth_rows_per_pos=11, G=2, T_kv=64)), 0) == 1
     assert lib.moda_b200_resolve_path(r(_prob(L=3, depth_rows_per_pos=11, G=2, T_kv=64, path=2)), 0) == -10

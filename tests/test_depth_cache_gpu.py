@@ -37,7 +37,7 @@ def _call(M, mode, q, k, v, ck, cv, G):
 
 @pytest.mark.parametrize("mode,B,T,H,D,G,n_layers", [
     (mo.MODE_NONCAUSAL, 2, 197, 3, 64, 1, 4),       # DeiT-like: own-position depth through the bandwidth kernels
-    (mo.MODE_CAUSAL, 1, 300, 2, 128, 4, 5),         # tcgen05 kernels, 5-D depth maps (L = 1, 2, 4) and mma.sync (L = 3)
+    (mo.MODE_CAUSAL, 1, 300, 2, 128, 4, 5),         # tcgen05 kernels, 5-D depth maps; L = 3 leaves tiles unfilled
     (mo.MODE_CHUNK_VISIBLE, 2, 160, 2, 64, 2, 3),
     (mo.MODE_CAUSAL, 1, 100, 2, 128, 1, 3),
 ])
@@ -76,9 +76,9 @@ def test_layer_stack_matches_rebuilt_cache_and_oracle(built_library, mode, B, T,
         kv.append((k, v))
     loss_b.backward()
     for i, ((oa, la), (ob, lb)) in enumerate(zip(outs_a, outs_b)):
-        # Layer i reads i cached layers.  Where both flows run the same kernels (the tcgen05 kernels
-        # read an in-place cache only when the layer count divides their 32-row boxes; the other
-        # counts fall to the mma.sync kernels) the arithmetic is the same and so are the bits.
+        # Layer i reads i cached layers.  Where both flows walk the same tiles (a tile of an in-place
+        # cache holds whole positions, so a layer count that does not divide its rows ends it early)
+        # the arithmetic is the same and so are the bits.
         same_kernels = D == 64 and G == 1 or i == 0 or 32 % i == 0 or i == n_layers - 1
         if same_kernels:
             assert torch.equal(oa, ob) and torch.equal(la, lb), f"layer {i}"
@@ -107,7 +107,7 @@ def test_layer_stack_matches_rebuilt_cache_and_oracle(built_library, mode, B, T,
 
 def test_strided_cache_with_forced_tcgen05_path(built_library):
     """Forced tcgen05: a layer count that divides 32 runs on 5-D tensor maps; one that does not is
-    refused (the default path serves it with the mma.sync kernels)."""
+    refused (the default path takes it)."""
     import moda_b200 as M
     dev = torch.device("cuda", 0)
     B, T, H, D, G = 1, 200, 2, 128, 2
