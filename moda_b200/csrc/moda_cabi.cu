@@ -281,15 +281,18 @@ int tc_forward(const Params& p, const moda_problem* prob, int n_sm, cudaStream_t
 }
 
 // Short sequences take the one-CTA-per-head backward where its kernel has a CTA for the whole problem (256
-// keys are what 16 warps hold in registers at D = 64; 512 query rows) and enough heads: a head is a serial
-// chain on one SM, which the tile kernels divide.  Estimates in us for 148 SMs, fitted to 22 shapes
+// keys are what 16 warps hold in registers at D = 64; 512 query rows), unless the tile kernels are much faster: a
+// head is a serial chain on one SM, which they divide.  Estimates in us for 148 SMs, fitted to 24 shapes
 // (T = 32..256, G = 1..8, causal and all keys) with 1 to 512 heads each:
 //   one round of CTAs  5 + blocks of 32 query rows x (2.2 + 0.07 warps, at least 8 / warps), under a causal
 //                      mask 0.01 of it less a warp, CTAs that share an SM a quarter longer
 //   tile kernels       8 + heads x (0.065 query tiles + 0.04 key tiles), at least 12 + 0.4 blocks
-// Short against tile kernels, causal, G = 1: T = 64 from 1 head 10.6, 12.2, 256 heads 13, 29; T = 197 1 head 25, 15, 64 heads
-// 25, 22, 128 heads 25, 35, 192 heads 46, 49, 512 heads 92, 114; T = 256, G = 2: 1 head 50, 19, 128 heads 51, 55,
-// 256 heads 103, 101.
+// The tile kernels are two launches more, 5 us for the calling thread, whose own time for a backward is some 45 us:
+// what the GPU takes below that nobody waits for where calls follow one another (eight heads, forward and
+// backward through autograd: T = 197 88 us short, 92 with the tile kernels; T = 128 67 and 72).
+// Short against tile kernels on the GPU, causal, G = 1: T = 64 from 1 head 10.6, 12.2, 256 heads 13, 29; T = 197 1 head 25, 15,
+// 128 heads 25, 35, 192 heads 46, 49, 512 heads 92, 114; G = 2, T = 256: 1 head 50, 19, 128 heads 51, 55, 192 heads 99,
+// 78; G = 8, T = 64: 16 heads 49, 18, 256 heads 57, 78.
 bool use_short_bwd(const moda_problem* att, int n_sm) {
   if (!(att->path == MODA_PATH_AUTO && att->mode != MODA_DEPTH_ONLY && att->D == shortseq::kD && att->L == 0 &&
         att->T_kv <= shortseq::kMaxKeys && (int64_t)att->T_kv * att->G <= 2 * shortseq::kMaxKeys && (int64_t)att->B * att->H <= 0x7fffffff))
@@ -302,7 +305,8 @@ bool use_short_bwd(const moda_problem* att, int n_sm) {
   if (att->mode != MODA_NONCAUSAL) round_us *= 1 - 0.01 * warps;
   if (per_sm > 1 && heads > n_sm) round_us *= 1.25;
   const double per_head = (0.065 * ((T_q + 127) / 128) + 0.04 * ((att->T_kv + 127) / 128)) * 148 / n_sm;
-  return 2 + rounds * round_us < std::max(12 + 0.4 * blocks, 8 + heads * per_head);
+  const double short_us = 2 + rounds * round_us, tile_us = std::max(12 + 0.4 * blocks, 8 + heads * per_head);
+  return short_us < 45 || short_us < tile_us + 5;
 }
 template <typename T>
 int short_bwd(const Params& p, cudaStream_t st) {

@@ -17,7 +17,7 @@
 // takes the statistics launch and its pass over o and dO away.
 // What bounds it now is the chain from block to block of its one CTA an SM (13 warps at T = 197: issue slots 31 %
 // busy, tensor pipe 24 %, most stalls at the block's barrier and on dependent instructions), which is why it
-// has no advantage beyond a few hundred keys, nor with few heads (use_short_bwd).  1536 heads (B = 256, H = 6),
+// has no advantage beyond a few hundred keys, nor on the GPU alone with few heads (use_short_bwd).  1536 heads (B = 256, H = 6),
 // T = 197: statistics + dq + dk/dv 404 us -> 351 us; 384 heads: 122 -> 97 us a layer.
 #pragma once
 #include "simt_mma_kernels.cuh"

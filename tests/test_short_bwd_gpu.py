@@ -55,8 +55,8 @@ def _kernels(call):
                                         ("causal", 170, 3, 0), ("chunk", 128, 4, 0), ("chunk", 64, 8, 0), ("chunk", 33, 2, 0),
                                         ("all", 13, 3, 0)])
 def test_short_backward_of_many_heads(built_library, mode, T, G, L, dt):
-    """Enough heads for the one-CTA-per-head kernel (the shapes above it are too few and take the tile kernels
-    from T = 64 on), in every mode and with query groups that do and do not divide a block of 32 rows."""
+    """Heads enough for the one-CTA-per-head kernel whatever the length, in every mode and with query groups that do
+    and do not divide a block of 32 rows."""
     import moda_b200 as M
     from moda_b200 import ops
     B, H, D = (70, 2, 64) if T >= 170 else (64, 4, 64)
@@ -76,8 +76,8 @@ def test_short_backward_of_many_heads(built_library, mode, T, G, L, dt):
     assert M.device_status() == 0
 
 
-@pytest.mark.parametrize("T,G,heads,short", [(64, 1, 4, True), (197, 1, 64, False), (197, 1, 128, True), (256, 2, 1, False),
-                                             (256, 2, 192, False), (197, 1, 384, True), (64, 8, 16, False)])
+@pytest.mark.parametrize("T,G,heads,short", [(64, 1, 4, True), (197, 1, 8, True), (197, 1, 128, True), (256, 2, 1, False),
+                                             (256, 2, 192, False), (197, 1, 384, True), (128, 4, 16, False)])
 def test_few_heads_take_the_tile_kernels(built_library, T, G, heads, short):
     from moda_b200 import ops
     q, k, dout = [torch.randn(heads, n, 1, 64, device="cuda", dtype=torch.bfloat16) for n in (T * G, T, T * G)]
